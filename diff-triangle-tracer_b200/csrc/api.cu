@@ -127,6 +127,10 @@ float* cache_colors_of(void* cache, int k, long long rays, long long cap) {
                                   (size_t)(k + 2) * 8 * (size_t)cap);
 }
 
+int shade_mode(const tt_tracer* h) {
+  return h->cfg.exact_adjoint ? tt::kShadeExact : (h->cfg.reference_arithmetic ? tt::kShadeRefArith : tt::kShadeRef);
+}
+
 int check_sh(tt_tracer* h, const float* shs, int deg, int M, int P, const float* cols = nullptr) {
   if (cols && !shs) return TT_OK;  // precomputed colours in place of SH
   TT_REQUIRE(h, deg >= 0 && deg <= 3, "sh_degree must be in [0, 3]");
@@ -161,8 +165,7 @@ int tt_create(const tt_config* cfg, tt_tracer** out) {
       (e = cudaDeviceGetAttribute(&h->num_sms, cudaDevAttrMultiProcessorCount, h->device)) != cudaSuccess ||
       (e = h->scratch.reserve(128)) != cudaSuccess || (e = cudaMemset(h->scratch.p, 0, 128)) != cudaSuccess ||
       (e = cudaEventCreate(&h->ev0)) != cudaSuccess || (e = cudaEventCreate(&h->ev1)) != cudaSuccess ||
-      (e = cudaEventCreate(&h->ev_mid)) != cudaSuccess ||
-      (e = tt::trace_init()) != cudaSuccess) {
+      (e = cudaEventCreate(&h->ev_mid)) != cudaSuccess) {
     delete h;
     return e == cudaErrorMemoryAllocation ? TT_ERR_OOM : TT_ERR_CUDA;
   }
@@ -171,9 +174,10 @@ int tt_create(const tt_config* cfg, tt_tracer** out) {
   h->sec_bwd_grid = h->num_sms * tt::sec_blocks_per_sm(1);
   h->sec_collect_grid = h->num_sms * tt::sec_blocks_per_sm(3);
   h->sec_collect0_grid = h->num_sms * tt::trace_blocks_per_sm(3, tt::kCfgPackets16);
-  if (tt_set_traversal(h, h->cfg.traversal, h->cfg.k, h->cfg.stack_depth) != TT_OK) {
+  const int rc = tt_set_traversal(h, h->cfg.traversal, h->cfg.k, h->cfg.stack_depth);
+  if (rc != TT_OK) {
     delete h;
-    return TT_ERR_INVALID;
+    return rc;
   }
   *out = h;
   return TT_OK;
@@ -193,6 +197,7 @@ int tt_set_traversal(tt_tracer* h, int traversal, int k, int stack_depth) {
     id = stack_depth == 24 ? tt::kCfgLanes24 : tt::kCfgLanes32;
   else
     id = k == 32 ? tt::kCfgPackets32 : tt::kCfgPackets16;
+  TT_CUDA(h, tt::trace_init(id, shade_mode(h)));
   h->cfg.traversal = traversal;
   h->cfg.k = k;
   h->cfg.stack_depth = stack_depth;
@@ -285,7 +290,7 @@ static tt::TraceParams base_params(tt_tracer* h) {
   std::memset(&p, 0, sizeof(p));
   p.bvh = h->bvh.view();
   p.tmin_inclusive = h->cfg.tmin_inclusive;
-  p.mode = h->cfg.exact_adjoint ? tt::kShadeExact : (h->cfg.reference_arithmetic ? tt::kShadeRefArith : tt::kShadeRef);
+  p.mode = shade_mode(h);
   p.variant = h->cfg.variant;
   p.cfg = h->cfg_id;
   p.count_work = h->count_work ? 1 : 0;

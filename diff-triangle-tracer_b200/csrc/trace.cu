@@ -7,11 +7,13 @@
 // Shape of the kernels:
 //  * persistent: every warp pulls 8x4-pixel tiles from an atomic counter until
 //    the image is done, so rays of very different depth complexity balance;
-//  * one ray per thread; the traversal stack (node reference + entry distance)
-//    lives in shared memory, strided by the block size (no bank conflicts);
-//  * k-buffer: the k nearest (t, primitive) pairs packed as 64-bit keys, kept
-//    sorted in shared memory (one column per lane) by insertion, the largest
-//    mirrored in a register;
+//  * one ray per thread. Warp packets walk the BVH together for the frustum
+//    around their rays; independent lanes each keep a traversal stack (node
+//    reference + entry distance) in shared memory, strided by the block size
+//    (no bank conflicts);
+//  * k-buffer: the k nearest (t, primitive) pairs packed as 64-bit keys in
+//    shared memory (one column per lane): sorted by insertion as hits arrive
+//    (lanes), or filled in any order and sorted at the end (packets);
 //  * the chunked march of the reference is reproduced exactly on top of the
 //    key stream: after every 16th visited hit the next query starts AT the
 //    last hit's t (closed interval, optixTrace) or strictly after it;
@@ -253,28 +255,166 @@ __device__ __forceinline__ void query(const BvhView& bvh, const RayW& r, unsigne
 }
 
 // ---------------------------------------------------------------- packets
-// Warp packet traversal for coherent rays (a warp = an 8x4-pixel tile of a
-// pinhole camera, whose rays all cross nearly the same BVH nodes). The warp
-// shares ONE stack in shared memory; an entry carries the node, the mask of
-// lanes whose ray hit its box and the smallest entry distance among them.
-// Every active lane tests its own ray (its own [t_lo, tmax] interval and
-// k-buffer) against the 8 children; ballots give each child's lane mask and
-// __reduce_min_sync its nearest entry distance; the triangles of hit leaf
-// children are tested at once by the lanes that entered them, and hit
-// interior children are ranked lane-parallel (lane c ranks child c) and
-// pushed far-to-near, so the stack holds interior nodes only. Control flow is
-// warp-uniform, so SIMT efficiency equals the fraction of lanes whose ray
-// still needs the node, and every node/triangle record is read once per warp.
-// Interior nodes only (leaf children are tested at their parent's visit):
-// a BVH8 of depth d needs at most ~7d entries.
-constexpr int kWarpStack = 96;
+// Warp packet traversal. The rays of a warp (an 8x4-pixel tile) are bounded by
+// one frustum, and the warp walks the BVH for the frustum instead of for each
+// ray: a lane tests one child box of one of four nodes, so 32 boxes cost what
+// one ray's test of a single child would. The triangles of entered leaves are
+// culled one a lane against the frustum, and the survivors, 32 at a time, one
+// a lane again, against every ray's line through the common origin (2 FMAs an
+// edge). Only the (triangle, ray) pairs left over run the watertight test, so
+// the hits do not depend on the culling: it only has to be conservative. A
+// triangle meets ~2 of a tile's 32 rays on the benchmark's clouds; testing
+// each against all rays, as the rays' own traversal did, wasted the rest.
+// Hits are appended to their ray's buffer in any order and the buffers sorted
+// at the end, all lanes at once; when one is full, all are sorted and cut back
+// to their K nearest, which then bound the rest.
+//
+// Traversal pass of 1M triangles, 4 views of 800^2, K = 32 (2.56M rays): 10.9
+// ms with a slab test per ray and child and an insert per hit, 6.4 with the
+// frustum alone (104k -> 41k instructions a tile), 5.3 with the hits deferred
+// and the pairs compacted (26k), 3.9 with the seven loads of a node wave in
+// flight at once (the test's short cuts had serialised them), 3.3 with 20
+// instead of 16 warps per SM (ray data shuffled instead of in shared memory).
+// What bounds it: latency (issue slots ~50 % busy at 20 warps), the node and
+// triangle loads' from L2 first.
+//
+// The frustum lives in the axes of the rays' dominant direction z: for z' (z
+// times the sign of the directions) in [z0, z1], every ray's u lies between
+// two lines u = off + slope z', and so does its v. Rays of one origin have the
+// lines of their extreme slopes; for others the chords between the extreme
+// positions at z0 and z1 bound them (the maximum of linear functions is
+// convex). Everything is padded by 2^-17 of the largest coordinate involved,
+// an order above the rounding of these lines (slopes are at most 2) and of the
+// watertight test itself.
+//
+// A wide frustum (coarse images, unrelated rays) holds many more triangles
+// than its rays hit. Such a warp takes its rays one by one: the frustum is
+// then the ray.
+constexpr int kWarpStack = 96;   // interior nodes: ref, nearest z'
+constexpr int kWarpQueue = 128;  // triangles of entered leaves (ring)
+constexpr int kWarpKept = 64;    // triangles the frustum kept (ring)
+constexpr int kWarpPairs = 64;   // (triangle, ray) pairs tested between two compactions
+constexpr int kSpare = 4;        // slots of a ray's buffer beyond its K keys
 
 struct WarpStack {
+  float4* slope;    // [16]: (a, a, b, b) of two rays: du/dz', dv/dz'
   uint32_t* ref;
-  unsigned* mask;
-  float* tmin;
-  unsigned* cnt;  // kWCounters words: the warp's traversal counters
+  float* z;
+  uint32_t* queue;
+  uint32_t* kept;
+  unsigned short* pair;
+  int* hits;        // [32] hits found so far, those past a full buffer included
+  unsigned* cnt;    // kWCounters words: the warp's traversal counters
+  float* scene;     // root box lo[3], hi[3], mean triangle extent
 };
+constexpr size_t kWarpBytes = 16 * 16 + kWarpStack * 8 + kWarpQueue * 4 + kWarpKept * 4 + kWarpPairs * 2 + 32 * 4 +
+                              kWCounters * 4 + 8 * 4;
+
+// Warp-wide minimum / maximum (NaN operands are ignored).
+__device__ __forceinline__ float warp_min(float v) {
+  float r;
+  asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+__device__ __forceinline__ float warp_max(float v) {
+  float r;
+  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+
+// Once per warp: the scene's box and the mean extent of 32 sampled triangles,
+// for the rule that decides between a packet and single rays.
+__device__ __forceinline__ void warp_scene(const BvhView& bvh, const WarpStack& ws) {
+  if (!bvh.has_root) return;
+  const int lane = threadIdx.x & 31;
+  const float* nd = reinterpret_cast<const float*>(bvh.nodes) + (lane & 7);
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const float lo = warp_min(__ldg(nd + 16 * a)), hi = warp_max(__ldg(nd + 16 * a + 8));
+    if (lane == 0) {
+      ws.scene[a] = lo;
+      ws.scene[3 + a] = hi;
+    }
+  }
+  const float4* tr = bvh.tris + 3 * (size_t)(((long long)lane * bvh.P) >> 5);
+  const float4 a = __ldg(tr), b = __ldg(tr + 1), c = __ldg(tr + 2);
+  float e = max3f(a.x, b.x, c.x) - min3f(a.x, b.x, c.x) + max3f(a.y, b.y, c.y) - min3f(a.y, b.y, c.y) +
+            max3f(a.z, b.z, c.z) - min3f(a.z, b.z, c.z);
+#pragma unroll
+  for (int s = 16; s > 0; s >>= 1) e += __shfl_xor_sync(0xFFFFFFFFu, e, s);
+  if (lane == 0) ws.scene[6] = e * (1.0f / 96.0f);
+  __syncwarp();
+}
+
+// A packet is taken when the triangles its frustum holds number at most
+// kPacketMin + kPacketRatio times those its rays meet. Forwards of pinhole
+// images (ms; as packets / ray by ray): 1M triangles 128^2 3.5 / 5.8, 256^2
+// 1.7 / 5.7; 3M triangles 64^2 22.0 / 9.2, 128^2 8.5 / 9.3, 256^2 3.9 / 9.8;
+// 616k triangles 31 x 38 21.2 / 3.5; 100k triangles 64^2 0.6 / 1.0.
+#ifndef TT_PACKET_MIN
+#define TT_PACKET_MIN 1024.0f
+#endif
+#ifndef TT_PACKET_RATIO
+#define TT_PACKET_RATIO 2.5f
+#endif
+
+// Sorts the first n keys of a lane's column, of which the first `done` are in
+// order (insertion: traversal finds hits nearly in order).
+__device__ __forceinline__ void kb_sort(unsigned long long* kb, int stride, int done, int n) {
+  for (int i = max(done, 1); i < n; ++i) {
+    const unsigned long long key = kb[i * stride];
+    int j = i;
+    for (; j > 0; --j) {
+      const unsigned long long prev = kb[(j - 1) * stride];
+      if (prev <= key) break;
+      kb[j * stride] = prev;
+    }
+    if (j != i) kb[j * stride] = key;
+  }
+}
+
+// The rays (bits, ray i of the packet in bit i) that may hit a triangle, given
+// as its vertices relative to the common origin in (u, v, z'): all three edge
+// planes through the origin have the ray on the inner side, up to 2^-18 of
+// |vertex| |edge| (L1 norms), an order above the rounding of both this test
+// and the watertight one for slopes of at most 2. An edge-on triangle, whose
+// side is in doubt, meets every ray.
+__device__ __forceinline__ unsigned rays_meeting(const float4* slope, float Au, float Av, float Az, float Bu, float Bv,
+                                                 float Bz, float Cu, float Cv, float Cz) {
+  const float kMargin = 3.814697265625e-6f;
+  const float abu = Bu - Au, abv = Bv - Av, abz = Bz - Az;
+  const float bcu = Cu - Bu, bcv = Cv - Bv, bcz = Cz - Bz;
+  const float cau = Au - Cu, cav = Av - Cv, caz = Az - Cz;
+  const float la = fabsf(Au) + fabsf(Av) + fabsf(Az), lb = fabsf(Bu) + fabsf(Bv) + fabsf(Bz),
+              lc = fabsf(Cu) + fabsf(Cv) + fabsf(Cz);
+  const float eab = fabsf(abu) + fabsf(abv) + fabsf(abz), ebc = fabsf(bcu) + fabsf(bcv) + fabsf(bcz),
+              eca = fabsf(cau) + fabsf(cav) + fabsf(caz);
+  // edge planes: n = vertex x edge
+  float n0u = fmaf(Bv, bcz, -(Bz * bcv)), n0v = fmaf(Bz, bcu, -(Bu * bcz)), n0z = fmaf(Bu, bcv, -(Bv * bcu));
+  float n1u = fmaf(Cv, caz, -(Cz * cav)), n1v = fmaf(Cz, cau, -(Cu * caz)), n1z = fmaf(Cu, cav, -(Cv * cau));
+  float n2u = fmaf(Av, abz, -(Az * abv)), n2v = fmaf(Az, abu, -(Au * abz)), n2z = fmaf(Au, abv, -(Av * abu));
+  const float det = fmaf(Au, n0u, fmaf(Av, n0v, Az * n0z));
+  if (!(fabsf(det) > kMargin * la * lb * ebc)) return 0xFFFFFFFFu;
+  const float s = det < 0.f ? -1.f : 1.f;
+  n0u *= s, n0v *= s, n1u *= s, n1v *= s, n2u *= s, n2v *= s;
+  n0z = fmaf(s, n0z, kMargin * lb * ebc);
+  n1z = fmaf(s, n1z, kMargin * lc * eca);
+  n2z = fmaf(s, n2z, kMargin * la * eab);
+  unsigned out = 0u;  // sign bits, ray 0 ends in bit 31
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const float4 ab = slope[i];
+    const float2 a = make_float2(ab.x, ab.y), b = make_float2(ab.z, ab.w);
+    const float2 e0 = __ffma2_rn(make_float2(n0u, n0u), a, __ffma2_rn(make_float2(n0v, n0v), b, make_float2(n0z, n0z)));
+    const float2 e1 = __ffma2_rn(make_float2(n1u, n1u), a, __ffma2_rn(make_float2(n1v, n1v), b, make_float2(n1z, n1z)));
+    const float2 e2 = __ffma2_rn(make_float2(n2u, n2u), a, __ffma2_rn(make_float2(n2v, n2v), b, make_float2(n2z, n2z)));
+    out = __funnelshift_l(__float_as_uint(min3f(e0.x, e1.x, e2.x)), out, 1);
+    out = __funnelshift_l(__float_as_uint(min3f(e0.y, e1.y, e2.y)), out, 1);
+  }
+  return __brev(~out);
+}
+
+constexpr float kPacketMin = TT_PACKET_MIN, kPacketRatio = TT_PACKET_RATIO;
 
 template <int K>
 __device__ __forceinline__ void packet_query(const BvhView& bvh, const RayW& r, bool want,
@@ -282,122 +422,308 @@ __device__ __forceinline__ void packet_query(const BvhView& bvh, const RayW& r, 
                                              WarpStack ws, float& t_drop, int* status, int count_work) {
   const unsigned full = 0xFFFFFFFFu;
   const int lane = threadIdx.x & 31;
-#pragma unroll
-  for (int i = 0; i < K; ++i) kb[i * kstride] = kEmptyKey;
-  int kb_n = 0;
+  const unsigned lt = (1u << lane) - 1u;
   t_drop = INFINITY;
-  const unsigned act = __ballot_sync(full, want);
-  if (act == 0 || !bvh.has_root) return;
-  if (lane == 0) ws.cnt[kWQueries] += __popc(act);
-  const float t_lo = want ? key_t(key_min) : 0.f;
-  float tmax = want ? t_hi : -1.0f;  // a lane without a query never passes a test
-  const int nx = r.ix >= 0.f ? 0 : 2, ny = r.iy >= 0.f ? 4 : 6, nz = r.iz >= 0.f ? 8 : 10;
-  // the rays of a packet nearly always share the watertight axis permutation:
-  // then the triangle tests use it as a compile-time constant
-  const int pk = perm_pack(r);
-  const int pk0 = __shfl_sync(full, pk, __ffs(act) - 1);
-  const int wperm = __all_sync(full, !want || pk == pk0) ? pk0 : -1;
-  if (lane == 0) {
-    ws.ref[0] = 0u;
-    ws.mask[0] = act;
-    ws.tmin[0] = 0.f;
+  float tmax = t_hi;
+  int kb_n = 0;  // leading keys of this lane's buffer that are in order
+  const float dm = max3f(fabsf(r.dx), fabsf(r.dy), fabsf(r.dz));
+  // a ray with a NaN, an infinity or no direction hits nothing
+  const bool usable = want && bvh.has_root && dm > 0.f &&
+                      fabsf(r.ox) + fabsf(r.oy) + fabsf(r.oz) + fabsf(r.dx) + fabsf(r.dy) + fabsf(r.dz) < INFINITY;
+  {
+    const unsigned asked = __ballot_sync(full, want);
+    if (lane == 0) ws.cnt[kWQueries] += __popc(asked);
   }
-  __syncwarp();
-  int sp = 1;
-  for (int steps = 0; sp > 0; ++steps) {
-    if (steps > kMaxSteps) {
-      if (lane == 0) atomicOr(status, kStatusTimeout);
-      break;
-    }
-    --sp;
-    const uint32_t ref = ws.ref[sp];
-    const float emin = ws.tmin[sp];
-    // lanes whose interval now ends before the entry's nearest distance drop out
-    const unsigned m = ws.mask[sp] & __ballot_sync(full, tmax >= emin);
-    __syncwarp();
-    if (m == 0) continue;
-    if (!TT_IN_BOUNDS(status, ref < (uint32_t)bvh.wide_cap)) continue;  // ref is the same in every lane
-    const bool on = (m >> lane) & 1u;
-    if (count_work && lane == 0) {
-      ws.cnt[kWNodes] += __popc(m);
-      ws.cnt[kWWarpNodes] += 1u;
-    }
-    const float4* nd = bvh.nodes + (size_t)ref * kNodeF4;
-    // lane c (c < 8) will push child c: fetch its reference with the boxes
-    const uint32_t my_ref = lane < 8 ? __ldg(reinterpret_cast<const uint32_t*>(nd + 12) + lane) : kEmptyRef;
-    float tn[8], tf[8];
-    slab8(nd, nx, ny, nz, r, t_lo, tmax, tn, tf);
-    // lane c (c < 8) collects child c: the mask of lanes entering it and
-    // their nearest entry distance
-    unsigned mymask = 0u;
-    float mine = INFINITY;
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      const bool hit = on && tn[c] <= tf[c];
-      const unsigned cm = __ballot_sync(full, hit);
-      const unsigned cmin = __reduce_min_sync(full, hit ? __float_as_uint(tn[c]) : 0x7F800000u);
-      if (lane == c) {
-        mymask = cm;
-        mine = __uint_as_float(cmin);
+  ws.hits[lane] = 0;
+  bool single = false;
+  for (unsigned rest = __ballot_sync(full, usable); rest != 0u;) {
+    const unsigned G = single ? (rest & (0u - rest)) : rest;
+    const int lead = __ffs(G) - 1;
+    const bool in = (G >> lane) & 1u;
+    const int kz = (__shfl_sync(full, r.perm, lead) >> 4) & 3;
+    const float sg = __shfl_sync(full, sel3(r.dx, r.dy, r.dz, kz), lead) < 0.f ? -1.f : 1.f;
+    const float dk = sg * sel3(r.dx, r.dy, r.dz, kz);
+    const float oz = sg * sel3(r.ox, r.oy, r.oz, kz);
+    float z0, z1, pad, oU1, oU0, oV1, oV0, sU1, sU0, sV1, sV0;
+    bool common;
+    {
+      const float ou = sel3(r.oy, r.oz, r.ox, kz), ov = sel3(r.oz, r.ox, r.oy, kz);
+      bool packet = __all_sync(full, !in || dk >= 0.5f * dm);
+      const float a = sel3(r.dy, r.dz, r.dx, kz) / dk, b = sel3(r.dz, r.dx, r.dy, kz) / dk;
+      const float rl = ws.scene[kz], rh = ws.scene[3 + kz];
+      z0 = fmaxf(warp_min(in ? fmaf(key_t(key_min), dk, oz) : INFINITY), sg > 0.f ? rl : -rh);
+      z1 = fminf(warp_max(in ? fmaf(tmax, dk, oz) : -INFINITY), sg > 0.f ? rh : -rl);
+      float m = fmaxf(warp_max(in ? max3f(fabsf(ou), fabsf(ov), fabsf(oz)) : 0.f), fmaxf(fabsf(z0), fabsf(z1)));
+      const float ou_l = __shfl_sync(full, ou, lead), ov_l = __shfl_sync(full, ov, lead),
+                  oz_l = __shfl_sync(full, oz, lead);
+      common = __all_sync(full, !in || (ou == ou_l && ov == ov_l && oz == oz_l));
+      if (common) {
+        sU1 = warp_max(in ? a : -INFINITY);
+        sU0 = warp_min(in ? a : INFINITY);
+        sV1 = warp_max(in ? b : -INFINITY);
+        sV0 = warp_min(in ? b : INFINITY);
+        oU1 = fmaf(-sU1, oz_l, ou_l);
+        oU0 = fmaf(-sU0, oz_l, ou_l);
+        oV1 = fmaf(-sV1, oz_l, ov_l);
+        oV0 = fmaf(-sV0, oz_l, ov_l);
+        float* sl = reinterpret_cast<float*>(ws.slope + (lane >> 1)) + (lane & 1);
+        sl[0] = in ? a : 0.f;
+        sl[2] = in ? b : 0.f;
+      } else {
+        const float zc = fmaxf(z1, z0 + fmaxf(m * 0.015625f, 1e-30f));  // chords over no shorter a range
+        const float ua = fmaf(a, z0 - oz, ou), ub = fmaf(a, zc - oz, ou);
+        const float va = fmaf(b, z0 - oz, ov), vb = fmaf(b, zc - oz, ov);
+        const float U1a = warp_max(in ? ua : -INFINITY), U0a = warp_min(in ? ua : INFINITY);
+        const float V1a = warp_max(in ? va : -INFINITY), V0a = warp_min(in ? va : INFINITY);
+        const float U1b = warp_max(in ? ub : -INFINITY), U0b = warp_min(in ? ub : INFINITY);
+        const float V1b = warp_max(in ? vb : -INFINITY), V0b = warp_min(in ? vb : INFINITY);
+        const float inv = 1.0f / (zc - z0);
+        sU1 = (U1b - U1a) * inv;
+        sU0 = (U0b - U0a) * inv;
+        sV1 = (V1b - V1a) * inv;
+        sV0 = (V0b - V0a) * inv;
+        oU1 = fmaf(-sU1, z0, U1a);
+        oU0 = fmaf(-sU0, z0, U0a);
+        oV1 = fmaf(-sV1, z0, V1a);
+        oV0 = fmaf(-sV0, z0, V0a);
+      }
+      m = fmaxf(m, fmaxf(max3f(fabsf(fmaf(sU1, z1, oU1)), fabsf(fmaf(sU0, z1, oU0)), fabsf(fmaf(sU1, z0, oU1))),
+                         max3f(fabsf(fmaf(sV1, z1, oV1)), fabsf(fmaf(sV0, z1, oV0)), fabsf(fmaf(sV1, z0, oV1)))));
+      pad = m * 7.62939453125e-6f;
+      if (!single) {
+        // triangles the frustum holds against those its rays meet, for
+        // triangles of the mean extent spread over the scene's box
+        const float zm = 0.5f * (z0 + z1);
+        const float w = fmaf(sU1 - sU0, zm, oU1 - oU0), h = fmaf(sV1 - sV0, zm, oV1 - oV0);
+        const float e = ws.scene[6];
+        const int ku = kz == 2 ? 0 : kz + 1, kv = kz == 0 ? 2 : kz - 1;
+        const float dens = (float)bvh.P / ((ws.scene[3 + ku] - ws.scene[ku]) * (ws.scene[3 + kv] - ws.scene[kv]));
+        packet = packet && (w + e) * (h + e) * dens <= fmaf(kPacketRatio * (float)__popc(G) * e * e, dens, kPacketMin);
+        if (!packet && __popc(G) > 1) {
+          single = true;
+          continue;
+        }
       }
     }
-    // Leaf children are tested right away by the lanes that entered them (a
-    // push and a pop saved per leaf); only interior children go on the stack.
-    const bool my_leaf = mymask != 0u && ref_is_leaf(my_ref);
-    for (unsigned lb = __ballot_sync(full, my_leaf); lb != 0u; lb &= lb - 1u) {
-      const int lc = __ffs(lb) - 1;
-      const uint32_t lref = __shfl_sync(full, my_ref, lc);
-      const unsigned lm = __shfl_sync(full, mymask, lc);  // lanes entering the leaf
-      const bool lon = (lm >> lane) & 1u;
-      const uint32_t first = leaf_first(lref), ntri = leaf_count(lref);
-      if (!TT_IN_BOUNDS(status, first + ntri <= (uint32_t)bvh.P)) continue;  // the same in every lane
-      if (count_work && lane == 0) ws.cnt[kWTris] += __popc(lm) * ntri;
-      with_perm(wperm, r, [&](const auto& pm) {
-        for (uint32_t j = 0; j < ntri; ++j) {
-          const float4* tr = bvh.tris + 3 * (size_t)(first + j);
-          const float4 a = __ldg(tr), b = __ldg(tr + 1), c = __ldg(tr + 2);
-          float t;
-          if (!lon || !isect_tri_p(r, pm, a, b, c, t)) continue;
-          if (!(t >= t_lo) || !(t <= tmax)) continue;
-          const unsigned long long key = hit_key(t, (uint32_t)__float_as_int(a.w));
-          if (key >= key_min && kb_accepts<K>(kb, kstride, key, kb_n)) {
-            if (kb_insert_smem<K>(kb, kstride, key, kb_n)) tmax = key_t(kb[(K - 1) * kstride]);
+    rest &= ~G;
+    z0 -= pad;
+    z1 += pad;
+    oU1 += pad;
+    oU0 -= pad;
+    oV1 += pad;
+    oV0 -= pad;
+    float zcur = z1;
+    if (lane == 0) {
+      ws.ref[0] = 0u;
+      ws.z[0] = z0;
+    }
+    __syncwarp();
+    int sp = z0 <= z1 ? 1 : 0, qh = 0, qn = 0, kh = 0, kn = 0;
+    for (int steps = 0;; ++steps) {
+      if (steps > kMaxSteps) {
+        if (lane == 0) atomicOr(status, kStatusTimeout);
+        break;
+      }
+      if (kn >= 32 || (sp == 0 && qn == 0 && kn > 0)) {
+        // ---- a batch of kept triangles, one a lane
+        const int n = min(kn, 32);
+        const uint32_t ti = ws.kept[(kh + lane) & (kWarpKept - 1)];
+        kh = (kh + n) & (kWarpKept - 1);
+        kn -= n;
+        float4 A = make_float4(0.f, 0.f, 0.f, 0.f), B = A, C = A;
+        unsigned m = 0u;  // rays the triangle may meet
+        const float cox = __shfl_sync(full, r.ox, lead), coy = __shfl_sync(full, r.oy, lead),
+                    coz = __shfl_sync(full, r.oz, lead);
+        if (lane < n) {
+          const float4* tr = bvh.tris + 3 * (size_t)ti;
+          A = __ldg(tr);
+          B = __ldg(tr + 1);
+          C = __ldg(tr + 2);
+          m = G;
+          if (common) {
+            const float ax = A.x - cox, ay = A.y - coy, az = A.z - coz;
+            const float bx = B.x - cox, by = B.y - coy, bz = B.z - coz;
+            const float cx = C.x - cox, cy = C.y - coy, cz = C.z - coz;
+            m &= rays_meeting(ws.slope, sel3(ay, az, ax, kz), sel3(az, ax, ay, kz), sg * sel3(ax, ay, az, kz),
+                              sel3(by, bz, bx, kz), sel3(bz, bx, by, kz), sg * sel3(bx, by, bz, kz),
+                              sel3(cy, cz, cx, kz), sel3(cz, cx, cy, kz), sg * sel3(cx, cy, cz, kz));
           }
         }
-      });
-    }
-    const unsigned pmask = my_leaf ? 0u : mymask;  // lane c: lanes entering interior child c
-    const int nh = __popc(__ballot_sync(full, pmask != 0u));
-    if (nh == 0) continue;
-    // rank among the entered children by entry distance: distances are >= 0,
-    // so their bit patterns order like the values; the low 3 bits make room
-    // for the slot (near-ties go by slot, which only affects the visit order)
-    const unsigned key = pmask != 0u ? ((__float_as_uint(mine) & ~7u) | (unsigned)lane) : 0xFFFFFFFFu;
-    int rank = 0;
+        if (count_work) {
+          const int tests = __reduce_add_sync(full, __popc(m));
+          if (lane == 0) ws.cnt[kWTris] += tests;
+        }
+        // the pairs left, compacted kWarpPairs at a time: a lane tests one
+        while (__any_sync(full, m != 0u)) {
+          int at = __popc(m);
 #pragma unroll
-    for (int c = 0; c < 8; ++c) rank += __shfl_sync(full, key, c) < key ? 1 : 0;
-    const int avail = kWarpStack - sp;
-    const int npush = nh < avail ? nh : avail;
-    if (pmask != 0u && rank < npush && TT_IN_BOUNDS(status, sp + npush - 1 - rank < kWarpStack)) {
-      const int pos = sp + npush - 1 - rank;  // nearest on top
-      ws.ref[pos] = my_ref;
-      ws.mask[pos] = pmask;
-      ws.tmin[pos] = mine;
-    }
-    if (nh > avail) {
-      // stack full: the farthest children are dropped; their rays only trust
-      // keys nearer than the dropped entry distance
-#pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        const unsigned m = __shfl_sync(full, pmask, c);
-        const float e = __shfl_sync(full, mine, c);
-        const int rk = __shfl_sync(full, rank, c);
-        if (m != 0u && rk >= npush && ((m >> lane) & 1u)) t_drop = fminf(t_drop, e);
+          for (int i = 1; i < 32; i <<= 1) {
+            const int v = __shfl_up_sync(full, at, i);
+            if (lane >= i) at += v;
+          }
+          const int pairs = min(__shfl_sync(full, at, 31), kWarpPairs);
+          for (at -= __popc(m); m != 0u && at < kWarpPairs; ++at, m &= m - 1u)
+            ws.pair[at] = (unsigned short)((lane << 5) | (__ffs(m) - 1));
+          __syncwarp();
+          for (int i = lane; i - lane < pairs; i += 32) {
+            const bool have = i < pairs;
+            const int pr = have ? ws.pair[i] : 0;
+            const int ray = pr & 31, tri = pr >> 5;
+            float4 a, b, c;
+            a.x = __shfl_sync(full, A.x, tri), a.y = __shfl_sync(full, A.y, tri), a.z = __shfl_sync(full, A.z, tri);
+            b.x = __shfl_sync(full, B.x, tri), b.y = __shfl_sync(full, B.y, tri), b.z = __shfl_sync(full, B.z, tri);
+            c.x = __shfl_sync(full, C.x, tri), c.y = __shfl_sync(full, C.y, tri), c.z = __shfl_sync(full, C.z, tri);
+            a.w = __shfl_sync(full, A.w, tri);
+            b.w = c.w = 0.f;
+            const unsigned long long lo = __shfl_sync(full, key_min, ray);
+            RayW q;
+            q.ox = __shfl_sync(full, r.ox, ray), q.oy = __shfl_sync(full, r.oy, ray), q.oz = __shfl_sync(full, r.oz, ray);
+            q.Sx = __shfl_sync(full, r.Sx, ray), q.Sy = __shfl_sync(full, r.Sy, ray), q.Sz = __shfl_sync(full, r.Sz, ray);
+            q.perm = __shfl_sync(full, r.perm, ray);
+            const float far = __shfl_sync(full, tmax, ray);
+            unsigned long long key = kEmptyKey;
+            if (have) {
+              float t;
+              if (isect_tri_p(q, PermRt(q.perm), a, b, c, t) && t >= 0.f && t <= far) {
+                key = hit_key(t, (uint32_t)__float_as_int(a.w));
+                if (key < lo) key = kEmptyKey;
+              }
+            }
+            while (__any_sync(full, key != kEmptyKey)) {
+              if (key != kEmptyKey) {
+                const int slot = atomicAdd(ws.hits + ray, 1);
+                if (slot < K + kSpare) {
+                  kb[slot * kstride + (ray - lane)] = key;
+                  key = kEmptyKey;
+                }
+              }
+              if (!__any_sync(full, key != kEmptyKey)) break;
+              // A buffer has no room: all are sorted and cut back to their K
+              // nearest, and what did not fit tries again if still near enough
+              __syncwarp();
+              const int n = min(ws.hits[lane], K + kSpare);
+              kb_sort(kb, kstride, kb_n, n);
+              kb_n = min(n, K);
+              ws.hits[lane] = kb_n;
+              if (kb_n == K) tmax = fminf(tmax, key_t(kb[(K - 1) * kstride]));
+              zcur = fminf(z1, warp_max(in ? fmaf(tmax, dk, oz) : -INFINITY) + pad);
+              __syncwarp();
+              const float nearer = __shfl_sync(full, tmax, ray);
+              if (key != kEmptyKey && key_t(key) > nearer) key = kEmptyKey;
+            }
+          }
+          __syncwarp();
+        }
+        __syncwarp();
+        continue;
       }
+      if (qn >= 32 || (sp == 0 && qn > 0)) {
+        // ---- a batch of leaf triangles, one a lane, against the frustum
+        const int n = min(qn, 32);
+        const uint32_t ti = ws.queue[(qh + lane) & (kWarpQueue - 1)];
+        qh = (qh + n) & (kWarpQueue - 1);
+        qn -= n;
+        bool keep = false;
+        if (lane < n) {
+          const float4* tr = bvh.tris + 3 * (size_t)ti;
+          const float4 A = __ldg(tr), B = __ldg(tr + 1), C = __ldg(tr + 2);
+          const float Au = sel3(A.y, A.z, A.x, kz), Av = sel3(A.z, A.x, A.y, kz), Az = sg * sel3(A.x, A.y, A.z, kz);
+          const float Bu = sel3(B.y, B.z, B.x, kz), Bv = sel3(B.z, B.x, B.y, kz), Bz = sg * sel3(B.x, B.y, B.z, kz);
+          const float Cu = sel3(C.y, C.z, C.x, kz), Cv = sel3(C.z, C.x, C.y, kz), Cz = sg * sel3(C.x, C.y, C.z, kz);
+          keep = (max3f(Az, Bz, Cz) >= z0) & (min3f(Az, Bz, Cz) <= zcur) &
+                 (min3f(fmaf(-sU1, Az, Au), fmaf(-sU1, Bz, Bu), fmaf(-sU1, Cz, Cu)) <= oU1) &
+                 (max3f(fmaf(-sU0, Az, Au), fmaf(-sU0, Bz, Bu), fmaf(-sU0, Cz, Cu)) >= oU0) &
+                 (min3f(fmaf(-sV1, Az, Av), fmaf(-sV1, Bz, Bv), fmaf(-sV1, Cz, Cv)) <= oV1) &
+                 (max3f(fmaf(-sV0, Az, Av), fmaf(-sV0, Bz, Bv), fmaf(-sV0, Cz, Cv)) >= oV0);
+        }
+        const unsigned km = __ballot_sync(full, keep);
+        if (keep) ws.kept[(kh + kn + __popc(km & lt)) & (kWarpKept - 1)] = ti;
+        kn += __popc(km);
+        __syncwarp();
+        continue;
+      }
+      if (sp == 0) break;
+      // ---- four nodes, eight children each: a lane tests one child box
+      const int take = sp > kWarpStack - 32 ? 1 : min(sp, 4);
+      const int q = lane >> 3;
+      bool on = q < take;
+      uint32_t ref = 0u;
+      if (on) {
+        ref = ws.ref[sp - 1 - q];
+        on = ws.z[sp - 1 - q] <= zcur && TT_IN_BOUNDS(status, ref < (uint32_t)bvh.wide_cap);
+      }
+      __syncwarp();
+      sp -= take;
+      if (count_work) {
+        const unsigned nodes = __popc(__ballot_sync(full, on)) >> 3;
+        if (lane == 0) {
+          ws.cnt[kWNodes] += nodes * __popc(G);
+          ws.cnt[kWWarpNodes] += nodes;
+        }
+      }
+      bool hit = false;
+      float za = 0.f;
+      uint32_t cref = kEmptyRef;
+      if (on) {
+        const float* nd = reinterpret_cast<const float*>(bvh.nodes + (size_t)ref * kNodeF4) + (lane & 7);
+        const int ku = kz == 2 ? 0 : kz + 1, kv = kz == 0 ? 2 : kz - 1;
+        const float zl = __ldg(nd + 16 * kz), zh = __ldg(nd + 16 * kz + 8);
+        const float ul = __ldg(nd + 16 * ku), uh = __ldg(nd + 16 * ku + 8);
+        const float vl = __ldg(nd + 16 * kv), vh = __ldg(nd + 16 * kv + 8);
+        cref = __float_as_uint(__ldg(nd + 48));
+        za = fmaxf(sg > 0.f ? zl : -zh, z0);
+        const float zb = fminf(sg > 0.f ? zh : -zl, zcur);
+        // (no short cuts: all loads in flight at once)
+        hit = (za <= zb) & (ul <= fmaxf(fmaf(sU1, za, oU1), fmaf(sU1, zb, oU1))) &
+              (uh >= fminf(fmaf(sU0, za, oU0), fmaf(sU0, zb, oU0))) &
+              (vl <= fmaxf(fmaf(sV1, za, oV1), fmaf(sV1, zb, oV1))) &
+              (vh >= fminf(fmaf(sV0, za, oV0), fmaf(sV0, zb, oV0)));
+      }
+      // leaves: their triangles go to the queue
+      const bool leaf = hit && ref_is_leaf(cref);
+      const uint32_t cnt = leaf ? leaf_count(cref) : 0u;
+      const unsigned b0 = __ballot_sync(full, cnt & 1u), b1 = __ballot_sync(full, cnt & 2u);
+      if (b0 | b1) {
+        const int at = qh + qn + __popc(b0 & lt) + 2 * __popc(b1 & lt);
+        const uint32_t first = leaf_first(cref);
+        if (leaf) {
+          const bool ok = TT_IN_BOUNDS(status, first + cnt <= (uint32_t)bvh.P);
+          ws.queue[at & (kWarpQueue - 1)] = ok ? first : 0u;
+          if (cnt > 1u) ws.queue[(at + 1) & (kWarpQueue - 1)] = ok ? first + 1u : 0u;
+          if (cnt > 2u) ws.queue[(at + 2) & (kWarpQueue - 1)] = ok ? first + 2u : 0u;
+        }
+        qn += __popc(b0) + 2 * __popc(b1);
+      }
+      // interior children: pushed farthest first, so the nearest are popped next
+      const bool inner = hit && !leaf;
+      const unsigned im = __ballot_sync(full, inner);
+      if (im != 0u) {
+        const int nh = __popc(im);
+        // distances from z0 are >= 0, so their bits order like the values; ties go by lane
+        const unsigned key = inner ? ((__float_as_uint(za - z0) & ~31u) | (unsigned)lane) : 0xFFFFFFFFu;
+        int rank = 0;
+        for (unsigned mm = im; mm != 0u; mm &= mm - 1u) rank += __shfl_sync(full, key, __ffs(mm) - 1) < key ? 1 : 0;
+        const int npush = min(nh, kWarpStack - sp);
+        if (inner && rank < npush) {
+          ws.ref[sp + npush - 1 - rank] = cref;
+          ws.z[sp + npush - 1 - rank] = za;
+        }
+        if (npush < nh) {
+          // stack full: the farthest children are dropped; the rays only trust
+          // keys nearer than the nearest of them
+          const float zd = warp_min(inner && rank >= npush ? za : INFINITY) - pad;
+          if (in) t_drop = fminf(t_drop, fmaxf((zd - oz) / dk * (1.0f - 1e-6f), 0.f));
+        }
+        sp += npush;
+      }
+      __syncwarp();
     }
     __syncwarp();
-    sp += npush;
   }
+  __syncwarp();
+  const int n = min(ws.hits[lane], K + kSpare);
+  kb_sort(kb, kstride, kb_n, n);
+  for (int i = n; i < K; ++i) kb[i * kstride] = kEmptyKey;
 }
 
 // ---------------------------------------------------------------- shading
@@ -1141,12 +1467,17 @@ __device__ __forceinline__ void drive(const TraceParams& p, const Smem& sm, Shad
 // packet query (all lanes whose ray is unfinished) and one shading pass until
 // every ray of the tile is done.
 __device__ __forceinline__ WarpStack warp_stack(unsigned char* base) {
-  const int w = threadIdx.x >> 5;
+  base += (size_t)(threadIdx.x >> 5) * kWarpBytes;
   WarpStack ws;
-  ws.ref = reinterpret_cast<uint32_t*>(base) + w * kWarpStack;
-  ws.mask = reinterpret_cast<unsigned*>(base + (size_t)(blockDim.x / 32) * kWarpStack * 4) + w * kWarpStack;
-  ws.tmin = reinterpret_cast<float*>(base + (size_t)(blockDim.x / 32) * kWarpStack * 8) + w * kWarpStack;
-  ws.cnt = reinterpret_cast<unsigned*>(base + (size_t)(blockDim.x / 32) * kWarpStack * 12) + w * kWCounters;
+  ws.slope = reinterpret_cast<float4*>(base);
+  ws.ref = reinterpret_cast<uint32_t*>(ws.slope + 16);
+  ws.z = reinterpret_cast<float*>(ws.ref + kWarpStack);
+  ws.queue = reinterpret_cast<uint32_t*>(ws.z + kWarpStack);
+  ws.kept = ws.queue + kWarpQueue;
+  ws.pair = reinterpret_cast<unsigned short*>(ws.kept + kWarpKept);
+  ws.hits = reinterpret_cast<int*>(ws.pair + kWarpPairs);
+  ws.cnt = reinterpret_cast<unsigned*>(ws.hits + 32);
+  ws.scene = reinterpret_cast<float*>(ws.cnt + kWCounters);
   return ws;
 }
 
@@ -1162,6 +1493,7 @@ __device__ __forceinline__ void drive_packets(const TraceParams& p, const Smem& 
   const bool replay = cache_replays<K>(p);
   const bool colors = cache_colors_on(p);
   if (lane < kWCounters) ws.cnt[lane] = 0u;
+  if constexpr (!kReplayOnly) warp_scene(p.bvh, ws);
   __syncwarp();
   WarpCounters wc{ws.cnt};
   for (;;) {
@@ -1263,7 +1595,7 @@ __device__ __forceinline__ void drive_packets(const TraceParams& p, const Smem& 
   }
 }
 
-template <int K>
+template <int K, bool kReplayOnly = false>
 __device__ __forceinline__ Smem packet_smem(unsigned char*& rest) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Smem s;
@@ -1272,7 +1604,7 @@ __device__ __forceinline__ Smem packet_smem(unsigned char*& rest) {
   s.st.ref = nullptr;
   s.st.tn = nullptr;
   s.st.stride = 0;
-  rest = smem_raw + (size_t)K * blockDim.x * 8;
+  rest = smem_raw + (size_t)(K + (kReplayOnly ? 0 : kSpare)) * blockDim.x * 8;
   return s;
 }
 
@@ -1302,10 +1634,11 @@ struct TraversalCfg<kCfgLanes24> {
   static constexpr int K = 16, SD = 24;
 };
 
-template <int CFG>
+template <int CFG, bool kReplayOnly = false>
 constexpr size_t smem_bytes_for() {
   using C = TraversalCfg<CFG>;
-  return C::packets ? (size_t)kTraceThreads * C::K * 8 + (size_t)(kTraceThreads / 32) * (kWarpStack * 12 + kWCounters * 4)
+  if (kReplayOnly) return (size_t)kTraceThreads * C::K * 8 + (size_t)(kTraceThreads / 32) * kWCounters * 4;
+  return C::packets ? (size_t)kTraceThreads * (C::K + kSpare) * 8 + (size_t)(kTraceThreads / 32) * kWarpBytes
                     : (size_t)kTraceThreads * (C::SD * 8 + kChunk * 8);
 }
 
@@ -1319,8 +1652,15 @@ __device__ __forceinline__ void run(const TraceParams& p, Shader& sh, Counters& 
   using C = TraversalCfg<CFG>;
   if constexpr (C::packets) {
     unsigned char* rest;
-    const Smem sm = packet_smem<C::K>(rest);
-    drive_packets<C::K, Shader, kReplayOnly>(p, sm, warp_stack(rest), sh, cnt);
+    const Smem sm = packet_smem<C::K, kReplayOnly>(rest);
+    WarpStack ws;
+    if constexpr (kReplayOnly) {
+      ws = WarpStack{};
+      ws.cnt = reinterpret_cast<unsigned*>(rest) + (threadIdx.x >> 5) * kWCounters;
+    } else {
+      ws = warp_stack(rest);
+    }
+    drive_packets<C::K, Shader, kReplayOnly>(p, sm, ws, sh, cnt);
   } else {
     drive<C::SD>(p, thread_smem<C::SD>(), sh, cnt);
   }
@@ -1497,7 +1837,7 @@ __global__ void __launch_bounds__(kTraceThreads, REPLAY ? kReplayBlocks : kMinBl
   if (p.fwd_pair && cache_complete<TraversalCfg<CFG>::K>(p) != REPLAY) return;
   cache_header<TraversalCfg<CFG>::K>(p, TraversalCfg<CFG>::packets && p.cache_colors != nullptr);
   Counters cnt;
-  FwdShader<MODE> sh(p, smem_bytes_for<CFG>());
+  FwdShader<MODE> sh(p, smem_bytes_for<CFG, REPLAY>());
   run<CFG, FwdShader<MODE>, REPLAY>(p, sh, cnt);
   // queries = those the march used, traversed here or replayed from the
   // collecting pass; hit_cache_replays counts the adjoint's replays only
@@ -1517,13 +1857,10 @@ __global__ void __launch_bounds__(kTraceThreads, REPLAY ? kReplayBlocks : kMinBl
 // no shading state or code the pass needs far fewer registers than the fused
 // kernel, so more warps per SM hide the latency of the node and triangle
 // loads, which is what bounds the traversal.
-// 6 blocks of 128 threads (80 registers, ~60 bytes of spills a thread since
-// the packet drivers keep their counters in shared memory): 24 warps per SM
-// against the fused kernel's 16. Measured on 1M triangles, 4 x 800^2 rays,
-// split forward storing two queries a ray: 15.4 ms at 6 blocks, 16.5 at 5
-// (95 registers, no spills), fused 19.0 (one run, same box). With the
-// counters in registers the 6-block build spilled ~170 bytes and was no
-// faster than 5 blocks.
+// Warps per SM decide it (the pass waits on loads). 32-hit packets: 5 blocks
+// of 128 threads, what their buffers leave of shared memory (3.3 ms on 1M
+// triangles, 4 x 800^2 rays; 3.9 at 4 blocks). 16-hit packets: 6 blocks at 80
+// registers (3M triangles at 1080p 2.6 ms; 2.8 at 5 and at 7, 3.3 at 4).
 #ifndef TT_COLLECT_BLOCKS
 #define TT_COLLECT_BLOCKS 6
 #endif
@@ -1541,7 +1878,7 @@ struct MarchShader {
 };
 
 template <int CFG>
-__global__ void __launch_bounds__(kTraceThreads, kCollectBlocks) k_collect(const __grid_constant__ TraceParams p) {
+__global__ void __launch_bounds__(kTraceThreads, CFG == kCfgPackets32 ? 5 : kCollectBlocks) k_collect(const __grid_constant__ TraceParams p) {
   cache_header<TraversalCfg<CFG>::K>(p, TraversalCfg<CFG>::packets && p.cache_colors != nullptr);
   Counters cnt;
   MarchShader sh(p);
@@ -2819,23 +3156,46 @@ int trace_blocks_per_sm(int which, int cfg) {
   return n > 0 ? n : 1;
 }
 
-// The exact-adjoint forward's accumulators take kExactSmemBytes after the
-// traversal's shared memory, which takes the lane configurations past the
-// default 48 KB of dynamic shared memory: opt those kernels in.
-cudaError_t trace_init() {
+// Opts the kernels of a traversal configuration and shading mode in to their
+// dynamic shared memory where it passes the default 48 KB: the buffers of
+// 32-hit packets, and the exact-adjoint forward's accumulators
+// (kExactSmemBytes after the traversal's). Only the configuration a handle
+// uses: an attribute call loads its kernel.
+template <int CFG, int MODE>
+cudaError_t opt_in_kernels() {
   cudaError_t e = cudaSuccess;
   auto opt_in = [&](const void* fn, size_t bytes) {
     if (e == cudaSuccess && bytes > 48 * 1024)
       e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   };
-  opt_in((const void*)k_forward<kCfgPackets16, kShadeExact>, smem_bytes_for<kCfgPackets16>() + kExactSmemBytes);
-  opt_in((const void*)k_forward<kCfgPackets32, kShadeExact>, smem_bytes_for<kCfgPackets32>() + kExactSmemBytes);
-  opt_in((const void*)k_forward<kCfgPackets16, kShadeExact, true>, smem_bytes_for<kCfgPackets16>() + kExactSmemBytes);
-  opt_in((const void*)k_forward<kCfgPackets32, kShadeExact, true>, smem_bytes_for<kCfgPackets32>() + kExactSmemBytes);
-  opt_in((const void*)k_forward<kCfgLanes24, kShadeExact>, smem_bytes_for<kCfgLanes24>() + kExactSmemBytes);
-  opt_in((const void*)k_forward<kCfgLanes32, kShadeExact>, smem_bytes_for<kCfgLanes32>() + kExactSmemBytes);
+  const size_t extra = MODE == kShadeExact ? kExactSmemBytes : 0;
+  opt_in((const void*)k_collect<CFG>, smem_bytes_for<CFG>());
+  opt_in((const void*)k_forward<CFG, MODE>, smem_bytes_for<CFG>() + extra);
+  opt_in((const void*)k_backward<CFG, MODE>, smem_bytes_for<CFG>());
   return e;
 }
+
+template <int MODE>
+cudaError_t trace_init_t(int cfg) {
+  switch (cfg) {
+    case kCfgPackets16: return opt_in_kernels<kCfgPackets16, MODE>();
+    case kCfgPackets32: return opt_in_kernels<kCfgPackets32, MODE>();
+    case kCfgLanes24: return opt_in_kernels<kCfgLanes24, MODE>();
+    default: return opt_in_kernels<kCfgLanes32, MODE>();
+  }
+}
+
+cudaError_t trace_init(int cfg, int mode) {
+  switch (mode) {
+    case kShadeExact: return trace_init_t<kShadeExact>(cfg);
+    case kShadeRefArith: return trace_init_t<kShadeRefArith>(cfg);
+    default: return trace_init_t<kShadeRef>(cfg);
+  }
+}
+
+// The replay-only builds' shared memory (keys and counters, and the exact
+// forward's accumulators) stays within the default.
+static_assert(smem_bytes_for<kCfgPackets32, true>() + kExactSmemBytes <= 48 * 1024, "replay builds need no opt-in");
 
 // Grid of a replay-only build: the traversing build's grid (SMs x its blocks
 // per SM) at the replay build's blocks per SM.
@@ -2846,9 +3206,9 @@ cudaError_t launch_forward_t(const TraceParams& p, int grid, cudaStream_t s) {
   const size_t extra = MODE == kShadeExact ? kExactSmemBytes : 0;
   if (p.fwd_pair) {
     if (p.cfg == kCfgPackets16)
-      k_forward<kCfgPackets16, MODE, true><<<replay_grid(grid), kTraceThreads, smem_bytes_for<kCfgPackets16>() + extra, s>>>(p);
+      k_forward<kCfgPackets16, MODE, true><<<replay_grid(grid), kTraceThreads, smem_bytes_for<kCfgPackets16, true>() + extra, s>>>(p);
     else
-      k_forward<kCfgPackets32, MODE, true><<<replay_grid(grid), kTraceThreads, smem_bytes_for<kCfgPackets32>() + extra, s>>>(p);
+      k_forward<kCfgPackets32, MODE, true><<<replay_grid(grid), kTraceThreads, smem_bytes_for<kCfgPackets32, true>() + extra, s>>>(p);
   }
   switch (p.cfg) {
     case kCfgPackets16: k_forward<kCfgPackets16, MODE><<<grid, kTraceThreads, smem_bytes_for<kCfgPackets16>() + extra, s>>>(p); break;
@@ -2863,9 +3223,9 @@ template <int MODE>
 cudaError_t launch_backward_t(const TraceParams& p, int grid, cudaStream_t s) {
   if (p.bwd_pair) {
     if (p.cfg == kCfgPackets16)
-      k_backward<kCfgPackets16, MODE, true><<<replay_grid(grid), kTraceThreads, smem_bytes_for<kCfgPackets16>(), s>>>(p);
+      k_backward<kCfgPackets16, MODE, true><<<replay_grid(grid), kTraceThreads, smem_bytes_for<kCfgPackets16, true>(), s>>>(p);
     else
-      k_backward<kCfgPackets32, MODE, true><<<replay_grid(grid), kTraceThreads, smem_bytes_for<kCfgPackets32>(), s>>>(p);
+      k_backward<kCfgPackets32, MODE, true><<<replay_grid(grid), kTraceThreads, smem_bytes_for<kCfgPackets32, true>(), s>>>(p);
   }
   switch (p.cfg) {
     case kCfgPackets16: k_backward<kCfgPackets16, MODE><<<grid, kTraceThreads, smem_bytes_for<kCfgPackets16>(), s>>>(p); break;

@@ -201,8 +201,9 @@ constexpr int kNumCfgs = 4;
 size_t trace_smem_bytes(int cfg);
 // Resident blocks per SM of the forward / adjoint / variant kernels.
 int trace_blocks_per_sm(int which /*0 forward, 1 adjoint, 2 variant, 3 collecting pass*/, int cfg);
-// once per handle: kernel attributes (dynamic shared memory opt-ins)
-cudaError_t trace_init();
+// kernel attributes (dynamic shared memory opt-ins) of a traversal
+// configuration and shading mode
+cudaError_t trace_init(int cfg, int mode);
 // Traversal-only pass that fills the hit cache with every query of the march.
 cudaError_t launch_collect(const TraceParams& p, int grid, cudaStream_t s);
 cudaError_t launch_forward(const TraceParams& p, int grid, cudaStream_t s);
