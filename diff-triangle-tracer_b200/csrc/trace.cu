@@ -1117,10 +1117,10 @@ __device__ __forceinline__ void clip_cursor(Cursor& c, const float* interval, in
 }
 
 // Visits the keys of one query (K keys, ascending, staged in shared memory)
-// in the reference's chunk order (forward.cu:99-154) and calls sh.visit(prim)
-// for each hit at or beyond the near plane; visit returns true to end the ray
-// (transmittance cut-off). Returns true when the ray is finished, else leaves
-// in `cur` where the next query starts.
+// in the reference's chunk order (forward.cu:99-154), each hit at or beyond the
+// near plane; consume_chunk calls sh.visit(prim) for it, which returns true to
+// end the ray (transmittance cut-off), and returns true when the ray is
+// finished, else leaves in `cur` where the next query starts.
 //
 // The reference re-traces after every 16th visited hit from last_hit_t
 // (closed interval: the hit(s) at last_hit_t come again) or just after it
@@ -1137,73 +1137,100 @@ __device__ __forceinline__ void clip_cursor(Cursor& c, const float* interval, in
 // in cnt.cont), or, if the interval held no hit at all, from the start of the
 // ray (a plain re-trace, cnt.restart). Either way every hit at or beyond
 // t_near is visited in the plain order.
-template <int K, class Shader, class Cnt>
-__device__ __forceinline__ bool consume_chunk(const Smem& sm, float t_drop, Cursor& cur, int tmin_inclusive,
-                                              int* status, Shader& sh, Cnt& cnt) {
+//
+// March: the position inside a query's buffer; next() moves to the next hit
+// to visit (its slot in m.i) or to the buffer's end.
+struct March {
+  unsigned long long last_key = 0;
+  int i = 0;
+  int boundaries = 0;
+  bool any = false;
+  bool visited = false;  // slot i was handed out by the last call
+};
+constexpr int kMarchVisit = 0;  // visit slot m.i
+constexpr int kMarchQuery = 1;  // the next query starts at cur.key_min
+constexpr int kMarchDone = 2;   // the ray is finished
+
+template <int K, bool kStopsAtClip, class Cnt>
+__device__ __forceinline__ int march_next(const Smem& sm, float t_drop, March& m, Cursor& cur, int tmin_inclusive, int P,
+                                          int* status, Cnt& cnt) {
   const bool truncated = t_drop < INFINITY;
   auto trusted = [&](unsigned long long key) {
     return key != kEmptyKey && !(truncated && key_t(key) >= t_drop);
   };
-  unsigned long long last_key = 0;
-  bool any = false;
-  // the stream ran out below cur.t_hi; `next` is where it would resume. A
-  // shader that cannot end a ray (the collecting pass) stops there too: the
+  // the stream ran out below cur.t_hi; `next` is where it would resume. The
+  // collecting pass (kStopsAtClip) cannot end a ray and stops there too: the
   // shading pass decides on continuations and re-traces.
   auto exhausted = [&](unsigned long long next) {
-    if (cur.t_hi >= kFar || Shader::kStopsAtClip) return true;
+    if (cur.t_hi >= kFar || kStopsAtClip) return kMarchDone;
     cur.t_hi = kFar;
-    if (!any && cur.chunks == 0) {
+    if (!m.any && cur.chunks == 0) {
       cur.key_min = first_key(tmin_inclusive);
       cnt.add_restart();
     } else {
       cur.key_min = next;
       cnt.add_cont();
     }
-    return false;
+    return kMarchQuery;
   };
-  int boundaries = 0;
-  sh.prepare();
-  int i = 0;
-  while (i < K) {
-    const unsigned long long key = sm.keys[i * sm.stride];
+  for (;;) {
+    if (m.visited) {
+      m.visited = false;
+      if (cur.ref_pos == kChunk) {
+        // the reference's next optixTrace starts at last_hit_t
+        cur.ref_pos = 0;
+        const unsigned long long tb = __float_as_uint(cur.last_hit_t);
+        const unsigned long long bound = tmin_inclusive ? (tb << 32) : ((tb + 1ull) << 32);
+        if (++m.boundaries > K) {  // 16+ hits at one t under the closed interval: no progress
+          atomicOr(status, kStatusTimeout);
+          return kMarchDone;
+        }
+        int j = 0;
+        while (j < K && trusted(sm.keys[j * sm.stride]) && sm.keys[j * sm.stride] < bound) ++j;
+        if (j < K && trusted(sm.keys[j * sm.stride])) {
+          m.i = j;  // continue inside the buffer
+          continue;
+        }
+        if (j < K && sm.keys[j * sm.stride] == kEmptyKey && !truncated) return exhausted(bound);
+        cur.key_min = bound;
+        return kMarchQuery;
+      }
+      ++m.i;
+    }
+    if (m.i >= K) break;
+    const unsigned long long key = sm.keys[m.i * sm.stride];
     if (!trusted(key)) break;
-    any = true;
-    last_key = key;
+    m.any = true;
+    m.last_key = key;
     const float t = key_t(key);
     // fmaxf(last + STEP_EPSILON, t) with the sum in double (forward.cu:111)
     cur.last_hit_t = fmaxf(__double2float_rn(__dadd_rn((double)cur.last_hit_t, kStepEps)), t);
     ++cur.ref_pos;
-    if (!TT_IN_BOUNDS(status, key_prim(key) < (uint32_t)sh.p.bvh.P)) return true;
-    if (t >= kNear && visit_slot(sh, key_prim(key), t, i, 0)) return true;
-    if (cur.ref_pos == kChunk) {
-      // the reference's next optixTrace starts at last_hit_t
-      cur.ref_pos = 0;
-      const unsigned long long tb = __float_as_uint(cur.last_hit_t);
-      const unsigned long long bound = tmin_inclusive ? (tb << 32) : ((tb + 1ull) << 32);
-      if (++boundaries > K) {  // 16+ hits at one t under the closed interval: no progress
-        atomicOr(status, kStatusTimeout);
-        return true;
-      }
-      int j = 0;
-      while (j < K && trusted(sm.keys[j * sm.stride]) && sm.keys[j * sm.stride] < bound) ++j;
-      if (j < K && trusted(sm.keys[j * sm.stride])) {
-        i = j;  // continue inside the buffer
-        continue;
-      }
-      if (j < K && sm.keys[j * sm.stride] == kEmptyKey && !truncated) return exhausted(bound);
-      cur.key_min = bound;
-      return false;
-    }
-    ++i;
+    if (!TT_IN_BOUNDS(status, key_prim(key) < (uint32_t)P)) return kMarchDone;
+    m.visited = true;
+    if (t >= kNear) return kMarchVisit;
   }
-  if (i < K && sm.keys[i * sm.stride] == kEmptyKey && !truncated)
-    return exhausted(any ? last_key + 1ull : cur.key_min);
-  if (!any) {
+  if (m.i < K && sm.keys[m.i * sm.stride] == kEmptyKey && !truncated)
+    return exhausted(m.any ? m.last_key + 1ull : cur.key_min);
+  if (!m.any) {
     atomicOr(status, kStatusStack);  // a truncated query that trusted nothing
-    return true;
+    return kMarchDone;
   }
-  cur.key_min = last_key + 1ull;
-  return false;
+  cur.key_min = m.last_key + 1ull;
+  return kMarchQuery;
+}
+
+template <int K, class Shader, class Cnt>
+__device__ __forceinline__ bool consume_chunk(const Smem& sm, float t_drop, Cursor& cur, int tmin_inclusive,
+                                              int* status, Shader& sh, Cnt& cnt) {
+  March m;
+  sh.prepare();
+  for (;;) {
+    const int r = march_next<K, Shader::kStopsAtClip>(sm, t_drop, m, cur, tmin_inclusive, sh.p.bvh.P, status, cnt);
+    if (r != kMarchVisit) return r == kMarchDone;
+    const unsigned long long key = sm.keys[m.i * sm.stride];
+    if (visit_slot(sh, key_prim(key), key_t(key), m.i, 0)) return true;
+  }
 }
 
 // View holding global tile `tile` (views are stored in tile order).
@@ -2031,10 +2058,16 @@ __global__ void __launch_bounds__(kTraceThreads, 4) k_variant(const __grid_const
 __device__ __forceinline__ void window_bwd(const Geom& g, float dL_dphi, float3 dL_dn3, float3 (&gv)[3]) {
   const float3 V[3] = {make_float3(0.f, 0.f, 0.f), g.e1, g.e2};
   gv[0] = gv[1] = gv[2] = make_float3(0.f, 0.f, 0.f);
+  unsigned at_max = 0u;
 #pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    if (fabsf(g.d[k] - g.phi_max) > 1e-6f) continue;
-    const float3 p1 = V[k], p2 = V[(k + 1) % 3], p3 = V[(k + 2) % 3];
+  for (int k = 0; k < 3; ++k) at_max |= fabsf(g.d[k] - g.phi_max) > 1e-6f ? 0u : 1u << k;
+  // nearly always one edge, but another one in every lane: the edge's vertices
+  // are selected instead of running one copy of the body per edge
+  for (; at_max != 0u; at_max &= at_max - 1u) {
+    const int k = __ffs(at_max) - 1;
+    const float3 p1 = k == 0 ? V[0] : (k == 1 ? V[1] : V[2]);
+    const float3 p2 = k == 0 ? V[1] : (k == 1 ? V[2] : V[0]);
+    const float3 p3 = k == 0 ? V[2] : (k == 1 ? V[0] : V[1]);
     const float3 aa = p1 - p3, bb = p2 - p3, cc = p1 - p2;
     const float3 n = fcross(aa, bb);
     const float3 ne = fcross(n, cc);
@@ -2046,12 +2079,12 @@ __device__ __forceinline__ void window_bwd(const Geom& g, float dL_dphi, float3 
     // ne = ((p1-p3) x (p2-p3)) x (p1-p2); Jacobians in the form of
     // vecmath.h:2808-2859, with v^T [u]x = v x u for the skew terms
     const float3 axb = n;
-    const float3 g1 = fdot(v, bb) * cc - fdot(bb, cc) * v + fcross(v, axb);
+    const float3 g1 = fdot(v, bb) * cc - fdot(bb, cc) * v + fcross(v, axb) - dL_dphi * Ne;
     const float3 g2 = fdot(aa, cc) * v - fdot(v, aa) * cc - fcross(v, axb);
     const float3 g3 = fdot(v, cc) * cc - fdot(cc, cc) * v;
-    gv[k] = gv[k] + g1 - dL_dphi * Ne;
-    gv[(k + 1) % 3] = gv[(k + 1) % 3] + g2;
-    gv[(k + 2) % 3] = gv[(k + 2) % 3] + g3;
+    gv[0] = gv[0] + (k == 0 ? g1 : (k == 1 ? g3 : g2));
+    gv[1] = gv[1] + (k == 0 ? g2 : (k == 1 ? g1 : g3));
+    gv[2] = gv[2] + (k == 0 ? g3 : (k == 1 ? g2 : g1));
   }
   {
     // n = (p1-p3) x (p2-p3): dn/dp1 = [p3-p2]x etc.; v^T [u]x = v x u
@@ -2148,9 +2181,106 @@ __device__ __noinline__ void window_bwd_exact(const Geom& g, float3 dir, float d
   }
 }
 
-// backward.cu:191-350: the same march, running C/N/D that include the current
-// hit, dL/dalpha from the final values, scattered gradients. EXACT: the full
-// chain rule of window_bwd_exact, and no gradient through a clamped alpha.
+// Upstream gradients of one ray, and what its adjoint needs of the forward's
+// outputs. backward.cu:296-312 forms dL/dalpha per channel as
+// g (T x - (X_final - X) / (1 - alpha)), X the channel's running sum of w x
+// including the current hit; summed over the channels that is
+// T q - (F - S) / (1 - alpha) with q = sum g x, S = sum w q and F = sum g X_final:
+// one running sum instead of seven.
+struct RayGrads {
+  float g0, g1, g2, gD, gN0, gN1, gN2;
+  float F;
+  // EXACT: middepth / distortion
+  float Df, Wf, distf, gMid, gDist;
+};
+
+template <bool EXACT>
+__device__ __forceinline__ RayGrads load_ray_grads(const ViewDesc& v, int pix) {
+  const int HW = v.H * v.W;
+  RayGrads r;
+  r.g0 = __ldg(v.dL_dpix + pix);
+  r.g1 = __ldg(v.dL_dpix + HW + pix);
+  r.g2 = __ldg(v.dL_dpix + 2 * HW + pix);
+  r.gD = __ldg(v.dL_doth + kDepthCh * HW + pix);
+  r.gN0 = __ldg(v.dL_doth + (kNormalCh + 0) * HW + pix);
+  r.gN1 = __ldg(v.dL_doth + (kNormalCh + 1) * HW + pix);
+  r.gN2 = __ldg(v.dL_doth + (kNormalCh + 2) * HW + pix);
+  r.Df = __ldg(v.others + kDepthCh * HW + pix);
+  r.F = r.g0 * __ldg(v.colors + pix) + r.g1 * __ldg(v.colors + HW + pix) + r.g2 * __ldg(v.colors + 2 * HW + pix) +
+        r.gD * r.Df + r.gN0 * __ldg(v.others + (kNormalCh + 0) * HW + pix) +
+        r.gN1 * __ldg(v.others + (kNormalCh + 1) * HW + pix) + r.gN2 * __ldg(v.others + (kNormalCh + 2) * HW + pix);
+  if (EXACT) {
+    r.Wf = __ldg(v.others + kAlphaCh * HW + pix);
+    r.distf = __ldg(v.others + kDistortionCh * HW + pix);
+    r.gMid = __ldg(v.dL_doth + kMidDepthCh * HW + pix);
+    r.gDist = __ldg(v.dL_doth + kDistortionCh * HW + pix);
+  }
+  return r;
+}
+
+// One blended hit's opacity and sigma gradients, scattered, and its vertex
+// gradients, given dL/dalpha (and, EXACT, dL/dt).
+template <int MODE>
+__device__ __forceinline__ void hit_grads(const TraceParams& p, uint32_t prim, const Geom& g, float3 d, float sig,
+                                          float opacity, float dL_dalpha, float dL_dt, float3 dL_dn, float3 (&gv)[3]) {
+  constexpr bool EXACT = MODE == kShadeExact;
+  const bool live = !EXACT || opacity * g.Cx < kAlphaMax;
+  const float dL_dC = live ? opacity * dL_dalpha : 0.0f;
+  if (live) red_add(p.d_opac + prim, dL_dalpha * g.Cx);
+  if (g.phi_final > 0.0f) red_add(p.d_sigma + prim, dL_dC * g.Cx * logf(g.phi_final));
+  const float dL_dphi = sig / g.phi_max * dL_dC * g.Cx;
+  if (EXACT)
+    window_bwd_exact(g, d, dL_dphi, dL_dC * sig * g.Cx, dL_dn, dL_dt, gv);
+  else
+    window_bwd(g, dL_dphi, dL_dn, gv);
+}
+
+// Scatters one blended hit's vertex and colour gradients.
+__device__ __forceinline__ void scatter_hit(const TraceParams& p, uint32_t prim, float w, float g0, float g1, float g2,
+                                            float3 raw, const float (&B)[16], const float3 (&gv)[3]) {
+  float* dt = p.d_tri + 3 * (size_t)__ldg(p.cumsum + prim);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    red_add(dt + 3 * k + 0, gv[k].x);
+    red_add(dt + 3 * k + 1, gv[k].y);
+    red_add(dt + 3 * k + 2, gv[k].z);
+  }
+  if (p.cols) {
+    red_add(p.d_cols + 3 * prim + 0, g0 * w);
+    red_add(p.d_cols + 3 * prim + 1, g1 * w);
+    red_add(p.d_cols + 3 * prim + 2, g2 * w);
+    return;
+  }
+  // SH: dRGB/dsh_k = B_k, masked where the colour was clamped at 0
+  const float e0 = raw.x < 0.f ? 0.f : g0 * w, e1 = raw.y < 0.f ? 0.f : g1 * w, e2 = raw.z < 0.f ? 0.f : g2 * w;
+  float* dsh = p.d_sh + (size_t)prim * p.M * 3;
+  const int n = sh_count(p.sh_degree);
+  if (p.M == 16 && n == 16) {
+#pragma unroll
+    for (int q = 0; q < 12; ++q) {
+      float v4[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int idx = 4 * q + j, k = idx / 3, ch = idx % 3;
+        v4[j] = B[k] * (ch == 0 ? e0 : (ch == 1 ? e1 : e2));
+      }
+      red_add4(dsh + 4 * q, v4[0], v4[1], v4[2], v4[3]);
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      if (k < n) {
+        red_add(dsh + 3 * k + 0, B[k] * e0);
+        red_add(dsh + 3 * k + 1, B[k] * e1);
+        red_add(dsh + 3 * k + 2, B[k] * e2);
+      }
+    }
+  }
+}
+
+// backward.cu:191-350: the same march, dL/dalpha from the final values and the
+// running sum, scattered gradients. EXACT: the full chain rule of
+// window_bwd_exact, and no gradient through a clamped alpha.
 template <int MODE>
 struct BwdShader {
   static constexpr bool EXACT = MODE == kShadeExact;
@@ -2159,13 +2289,11 @@ struct BwdShader {
   const ViewDesc* v;
   int pix;
   float3 o, d;
-  // per-ray finals and upstream gradients, loaded for each chunk (so they do
-  // not occupy registers during traversal)
-  float Cf0, Cf1, Cf2, Df, Nf0, Nf1, Nf2;
-  float g0, g1, g2, gD, gN0, gN1, gN2;
-  float C0, C1, C2, N0, N1, N2, D, T;
-  // EXACT: middepth / distortion (finals per chunk, running sum S, mid flag)
-  float Wf, distf, gMid, gDist, S;
+  // upstream gradients and finals, loaded for each chunk (so they do not
+  // occupy registers during traversal)
+  RayGrads r;
+  float S, T;
+  float Sd;  // EXACT: running sum of the distortion's w E
   bool mid_seen;
 
   __device__ explicit BwdShader(const TraceParams& params) : p(params) {}
@@ -2175,38 +2303,16 @@ struct BwdShader {
     pix = pixel;
     o = ro;
     d = rd;
-    C0 = C1 = C2 = N0 = N1 = N2 = D = 0.f;
-    T = 1.0f;
     S = 0.f;
+    T = 1.0f;
+    Sd = 0.f;
     mid_seen = false;
     return true;
   }
 
   __device__ __forceinline__ bool next(float3&, float3&) { return false; }
 
-  __device__ __forceinline__ void prepare() {
-    const int HW = v->H * v->W;
-    Cf0 = __ldg(v->colors + pix);
-    Cf1 = __ldg(v->colors + HW + pix);
-    Cf2 = __ldg(v->colors + 2 * HW + pix);
-    Df = __ldg(v->others + kDepthCh * HW + pix);
-    Nf0 = __ldg(v->others + (kNormalCh + 0) * HW + pix);
-    Nf1 = __ldg(v->others + (kNormalCh + 1) * HW + pix);
-    Nf2 = __ldg(v->others + (kNormalCh + 2) * HW + pix);
-    g0 = __ldg(v->dL_dpix + pix);
-    g1 = __ldg(v->dL_dpix + HW + pix);
-    g2 = __ldg(v->dL_dpix + 2 * HW + pix);
-    gD = __ldg(v->dL_doth + kDepthCh * HW + pix);
-    gN0 = __ldg(v->dL_doth + (kNormalCh + 0) * HW + pix);
-    gN1 = __ldg(v->dL_doth + (kNormalCh + 1) * HW + pix);
-    gN2 = __ldg(v->dL_doth + (kNormalCh + 2) * HW + pix);
-    if (EXACT) {
-      Wf = __ldg(v->others + kAlphaCh * HW + pix);
-      distf = __ldg(v->others + kDistortionCh * HW + pix);
-      gMid = __ldg(v->dL_doth + kMidDepthCh * HW + pix);
-      gDist = __ldg(v->dL_doth + kDistortionCh * HW + pix);
-    }
-  }
+  __device__ __forceinline__ void prepare() { r = load_ray_grads<EXACT>(*v, pix); }
 
   // colour rows of the current query's hit-cache entry (the forward's raw
   // colour of each blended hit), or nullptr: then the SH are evaluated
@@ -2243,83 +2349,27 @@ struct BwdShader {
     }
     const float c0 = p.cols ? raw.x : fmaxf(raw.x, 0.f), c1 = p.cols ? raw.y : fmaxf(raw.y, 0.f),
                 c2 = p.cols ? raw.z : fmaxf(raw.z, 0.f);
-    C0 += c0 * w;
-    C1 += c1 * w;
-    C2 += c2 * w;
-    N0 += g.n.x * w;
-    N1 += g.n.y * w;
-    N2 += g.n.z * w;
-    D += w * g.t;
-    // backward.cu:296-312; C/N/D already include this hit
+    const float q = r.g0 * c0 + r.g1 * c1 + r.g2 * c2 + r.gD * g.t + r.gN0 * g.n.x + r.gN1 * g.n.y + r.gN2 * g.n.z;
+    S += w * q;
     const float inv1a = 1.0f / (1.0f - alpha);
-    float dL_dalpha = g0 * (T * c0 - (Cf0 - C0) * inv1a) + g1 * (T * c1 - (Cf1 - C1) * inv1a) +
-                      g2 * (T * c2 - (Cf2 - C2) * inv1a);
-    dL_dalpha += gD * (T * g.t - (Df - D) * inv1a);
-    dL_dalpha += gN0 * (T * g.n.x - (Nf0 - N0) * inv1a) + gN1 * (T * g.n.y - (Nf1 - N1) * inv1a) +
-                 gN2 * (T * g.n.z - (Nf2 - N2) * inv1a);
-    float dL_dt = gD * w;
+    float dL_dalpha = T * q - (r.F - S) * inv1a;
+    float dL_dt = r.gD * w;
     if (EXACT) {
       // distortion: dD/dalpha_k = T_k E_k - (2 D_f - S_k) / (1 - alpha_k),
       // E_k = t^2 W_f - 2 t B_f + C_f, C_f = (D_f + B_f^2) / W_f; dD/dt_k = 2 w (t W_f - B_f)
-      const float Cf = Wf > 0.f ? (distf + Df * Df) / Wf : 0.f;
-      const float E = g.t * g.t * Wf - 2.0f * g.t * Df + Cf;
-      S += w * E;
-      dL_dalpha += gDist * (T * E - (2.0f * distf - S) * inv1a);
-      dL_dt += gDist * 2.0f * w * (g.t * Wf - Df);
+      const float Cf = r.Wf > 0.f ? (r.distf + r.Df * r.Df) / r.Wf : 0.f;
+      const float E = g.t * g.t * r.Wf - 2.0f * g.t * r.Df + Cf;
+      Sd += w * E;
+      dL_dalpha += r.gDist * (T * E - (2.0f * r.distf - Sd) * inv1a);
+      dL_dt += r.gDist * 2.0f * w * (g.t * r.Wf - r.Df);
       if (!mid_seen && test_T <= 0.5f) {
         mid_seen = true;
-        dL_dt += gMid;
+        dL_dt += r.gMid;
       }
     }
-    const bool live = !EXACT || opacity * g.Cx < kAlphaMax;
-    const float dL_dC = live ? opacity * dL_dalpha : 0.0f;
-    if (live) red_add(p.d_opac + prim, dL_dalpha * g.Cx);
-    if (g.phi_final > 0.0f) red_add(p.d_sigma + prim, dL_dC * g.Cx * logf(g.phi_final));
-    const float dL_dphi = sig / g.phi_max * dL_dC * g.Cx;
     float3 gv[3];
-    if (EXACT)
-      window_bwd_exact(g, d, dL_dphi, dL_dC * sig * g.Cx, make_float3(gN0 * w, gN1 * w, gN2 * w), dL_dt, gv);
-    else
-      window_bwd(g, dL_dphi, make_float3(gN0 * w, gN1 * w, gN2 * w), gv);
-    float* dt = p.d_tri + 3 * (size_t)__ldg(p.cumsum + prim);
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      red_add(dt + 3 * k + 0, gv[k].x);
-      red_add(dt + 3 * k + 1, gv[k].y);
-      red_add(dt + 3 * k + 2, gv[k].z);
-    }
-    if (p.cols) {
-      red_add(p.d_cols + 3 * prim + 0, g0 * w);
-      red_add(p.d_cols + 3 * prim + 1, g1 * w);
-      red_add(p.d_cols + 3 * prim + 2, g2 * w);
-      T = test_T;
-      return false;
-    }
-    // SH: dRGB/dsh_k = B_k, masked where the colour was clamped at 0
-    const float e0 = raw.x < 0.f ? 0.f : g0 * w, e1 = raw.y < 0.f ? 0.f : g1 * w, e2 = raw.z < 0.f ? 0.f : g2 * w;
-    float* dsh = p.d_sh + (size_t)prim * p.M * 3;
-    const int n = sh_count(p.sh_degree);
-    if (p.M == 16 && n == 16) {
-#pragma unroll
-      for (int q = 0; q < 12; ++q) {
-        float v4[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int idx = 4 * q + j, k = idx / 3, ch = idx % 3;
-          v4[j] = B[k] * (ch == 0 ? e0 : (ch == 1 ? e1 : e2));
-        }
-        red_add4(dsh + 4 * q, v4[0], v4[1], v4[2], v4[3]);
-      }
-    } else {
-#pragma unroll
-      for (int k = 0; k < 16; ++k) {
-        if (k < n) {
-          red_add(dsh + 3 * k + 0, B[k] * e0);
-          red_add(dsh + 3 * k + 1, B[k] * e1);
-          red_add(dsh + 3 * k + 2, B[k] * e2);
-        }
-      }
-    }
+    hit_grads<MODE>(p, prim, g, d, sig, opacity, dL_dalpha, dL_dt, make_float3(r.gN0 * w, r.gN1 * w, r.gN2 * w), gv);
+    scatter_hit(p, prim, w, r.g0, r.g1, r.g2, raw, B, gv);
     T = test_T;
     return false;
   }
@@ -2327,19 +2377,342 @@ struct BwdShader {
   __device__ __forceinline__ void end() {}
 };
 
-// The adjoint. REPLAY: the replay-only build (packet configurations), which
-// needs a complete hit cache. Given a cache, the host launches the two builds
-// back to back (p.bwd_pair): the replay-only one works when the cache is
-// complete, the traversing one otherwise, and the other returns at once;
-// the choice is read on the device, so nothing synchronises.
-template <int CFG, int MODE, bool REPLAY = false>
-__global__ void __launch_bounds__(kTraceThreads, REPLAY ? kReplayBlocks : kMinBlocks) k_backward(const __grid_constant__ TraceParams p) {
-  if (p.bwd_pair && cache_complete<TraversalCfg<CFG>::K>(p) != REPLAY) return;
+// The adjoint that marches ray by ray: re-traversing, or with the queries of
+// an incomplete hit cache. Given a cache, the packet configurations launch
+// k_adjoint first (p.bwd_pair): it works when the cache is complete and this
+// kernel otherwise, and the other returns at once; the choice is read on the
+// device, so nothing synchronises.
+template <int CFG, int MODE>
+__global__ void __launch_bounds__(kTraceThreads, kMinBlocks) k_backward(const __grid_constant__ TraceParams p) {
+  if (p.bwd_pair && cache_complete<TraversalCfg<CFG>::K>(p)) return;
   Counters cnt;
   BwdShader<MODE> sh(p);
-  run<CFG, BwdShader<MODE>, REPLAY>(p, sh, cnt);
+  run<CFG>(p, sh, cnt);
   const unsigned s = __reduce_add_sync(0xFFFFFFFFu, cnt.replays);
   if ((threadIdx.x & 31) == 0 && s != 0u) atomicAdd(p.stats + kStatReplays, (unsigned long long)s);
+}
+
+// Inclusive scans over the lanes of a segment (first lane `seg`).
+__device__ __forceinline__ float seg_product(float v, int lane, int seg) {
+#pragma unroll
+  for (int i = 1; i < 32; i <<= 1) {
+    const float u = __shfl_up_sync(0xFFFFFFFFu, v, i);
+    if (lane - i >= seg) v *= u;
+  }
+  return v;
+}
+__device__ __forceinline__ float seg_sum(float v, int lane, int seg) {
+#pragma unroll
+  for (int i = 1; i < 32; i <<= 1) {
+    const float u = __shfl_up_sync(0xFFFFFFFFu, v, i);
+    if (lane - i >= seg) v += u;
+  }
+  return v;
+}
+
+// The adjoint over a complete hit cache, a lane per hit instead of per ray.
+// Ray by ray, a warp's lanes run as many steps as its longest ray, 17 of 32
+// lanes at work on the benchmark's clouds, each step waiting on its gathers.
+// Here each ray's march only lists its next hits (kVisits a round); the lists
+// of the tile's rays are laid end to end and taken 32 at a time, and what a
+// hit needs of the ones before it on its ray, the transmittance and the sum
+// of w q, are two segmented scans, carried from one step to the next in
+// shared memory. A ray ends at the first hit whose product falls below the
+// cut-off.
+//
+// What bounds it then is L2's handling of the reductions: 23 a hit (12 of 16
+// bytes, the others of 4), each a request and a sector of its own when every
+// lane scatters its own hit. So the gradients are staged in shared memory and
+// the lanes regrouped: 12 neighbouring lanes add a hit's 192 bytes of SH
+// gradient and 9 its vertices, which the load/store unit merges into whole
+// sectors, ~5 requests and 10 sectors a hit.
+//
+// Measured (ms; ray by ray / a lane per hit / regrouped reductions): 1M
+// triangles, 4 views of 800^2, 28M blended hits 4.2 / 4.3 / 3.2; 3M triangles,
+// 16 views, 180M hits 39.0 / 38.6 / 22.1; exact adjoint of 200k triangles
+// 0.24 / 0.18 / 0.19. It issues on 46 % of cycles with L2 39 % and DRAM 16 %
+// busy: bound by instructions and their latency at 16 warps per SM.
+constexpr int kVisits = 6;
+
+struct AdjointMem {
+  float4* ray;          // [4][32]: o, gD | d, F | g, T | gN, S (T < 0: the ray has ended)
+  float4* exact;        // [2][32] EXACT: Df, Wf, distf, gDist | gMid, Sd
+  float* basis;         // [32][16] SH basis
+  float* stage;         // [32][8] e0 e1 e2 e0 e1, prim, ray | [32][9] vertex gradients, [32] first vertex
+  unsigned short* list; // [32 * kVisits]: ray << 8 | slot
+};
+template <int MODE>
+constexpr size_t adjoint_warp_bytes() {
+  return (size_t)32 * 16 * (4 + 4 + (MODE == kShadeExact ? 2 : 0)) + 32 * 10 * 4 + 32 * kVisits * 2;
+}
+template <int K, int MODE>
+constexpr size_t adjoint_smem() {
+  return (size_t)kTraceThreads * K * 8 + (size_t)(kTraceThreads / 32) * adjoint_warp_bytes<MODE>();
+}
+
+#ifndef TT_ADJOINT_BLOCKS
+#define TT_ADJOINT_BLOCKS 4
+#endif
+constexpr int kAdjointBlocks = TT_ADJOINT_BLOCKS;
+
+template <int K, int MODE>
+__global__ void __launch_bounds__(kTraceThreads, kAdjointBlocks) k_adjoint(const __grid_constant__ TraceParams p) {
+  if (!cache_complete<K>(p)) return;
+  constexpr bool EXACT = MODE == kShadeExact;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const unsigned full = 0xFFFFFFFFu;
+  const int lane = threadIdx.x & 31;
+  Smem sm;
+  sm.keys = reinterpret_cast<unsigned long long*>(smem_raw) + threadIdx.x;
+  sm.stride = blockDim.x;
+  AdjointMem am;
+  {
+    unsigned char* base = smem_raw + (size_t)K * blockDim.x * 8 + (threadIdx.x >> 5) * adjoint_warp_bytes<MODE>();
+    am.ray = reinterpret_cast<float4*>(base);
+    am.exact = am.ray + 4 * 32;
+    am.basis = reinterpret_cast<float*>(am.exact + (EXACT ? 2 * 32 : 0));
+    am.stage = am.basis + 16 * 32;
+    am.list = reinterpret_cast<unsigned short*>(am.stage + 32 * 10);
+  }
+  const bool colors = cache_colors_on(p);
+  const bool sh16 = !p.cols && p.M == 16 && p.sh_degree == 3;
+  const int row = p.cols ? 3 : 3 * sh_count(p.sh_degree);  // colour gradients of a hit
+  unsigned replays = 0;
+  Counters cnt;  // (interval continuations and re-traces are the forward's to count)
+  for (;;) {
+    int tile = 0;
+    if (lane == 0) tile = atomicAdd(p.work, 1);
+    tile = __shfl_sync(full, tile, 0);
+    if (tile >= p.ntiles) break;
+    const ViewDesc& v = p.views[find_view(p, tile)];
+    const int lt = tile - v.tile_begin;
+    const int px = (lt % v.ntx) * 8 + (lane & 7), py = (lt / v.ntx) * 4 + (lane >> 3);
+    bool active = px < v.W && py < v.H;
+    Cursor cur = first_cursor(p.tmin_inclusive);
+    long long ray_g = 0;
+    if (active) {
+      const int pix = py * v.W + px;
+      ray_g = v.ray_begin + pix;
+      const float3 o = make_float3(v.ray_o[3 * pix], v.ray_o[3 * pix + 1], v.ray_o[3 * pix + 2]);
+      const float3 d = make_float3(v.ray_d[3 * pix], v.ray_d[3 * pix + 1], v.ray_d[3 * pix + 2]);
+      if (v.interval) clip_cursor(cur, v.interval, v.H * v.W, pix);
+      const RayGrads r = load_ray_grads<EXACT>(v, pix);
+      am.ray[lane] = make_float4(o.x, o.y, o.z, r.gD);
+      am.ray[32 + lane] = make_float4(d.x, d.y, d.z, r.F);
+      am.ray[64 + lane] = make_float4(r.g0, r.g1, r.g2, 1.0f);
+      am.ray[96 + lane] = make_float4(r.gN0, r.gN1, r.gN2, 0.0f);
+      if (EXACT) {
+        am.exact[lane] = make_float4(r.Df, r.Wf, r.distf, r.gDist);
+        am.exact[32 + lane] = make_float4(r.gMid, 0.0f, 0.0f, 0.0f);
+      }
+      if (!p.cols) {
+        float B[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) B[i] = 0.f;
+        sh_basis(unit(d), p.sh_degree, B);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          reinterpret_cast<float4*>(am.basis + 16 * lane)[i] = make_float4(B[4 * i], B[4 * i + 1], B[4 * i + 2], B[4 * i + 3]);
+      }
+    }
+    uint32_t next = kNoEntry;
+    for (bool first = true; __any_sync(full, active); first = false) {
+      // the cache holds every query of every march
+      bool have = active && (first || cache_has<K>(p, next, cur.key_min));
+      if (active && !have) {
+        atomicOr(p.status, kStatusCacheMiss);
+        active = false;
+      }
+      replays += __popc(__ballot_sync(full, have));
+      float t_drop = INFINITY;
+      float* rows = nullptr;
+      int rstride = 0;
+      if (have) {
+        if (colors) rows = cache_color_rows<K>(p, first, ray_g, next, rstride);
+        t_drop = cache_get<K>(p, first, ray_g, next, sm, next);
+      }
+      March m;
+      bool marching = have;
+      while (__any_sync(full, marching)) {
+        // ---- each ray lists its next hits
+        unsigned long long slots = 0ull;
+        int count = 0, state = kMarchVisit;
+        while (marching && count < kVisits) {
+          state = march_next<K, false>(sm, t_drop, m, cur, p.tmin_inclusive, p.bvh.P, p.status, cnt);
+          if (state != kMarchVisit) break;
+          slots |= (unsigned long long)m.i << (8 * count);
+          ++count;
+        }
+        if (marching && state != kMarchVisit) {
+          marching = false;
+          if (state == kMarchDone) {
+            active = false;
+          } else if (++cur.chunks >= kMaxChunks) {
+            atomicOr(p.status, kStatusTimeout);
+            active = false;
+          }
+        }
+        int at = count;
+#pragma unroll
+        for (int i = 1; i < 32; i <<= 1) {
+          const int u = __shfl_up_sync(full, at, i);
+          if (lane >= i) at += u;
+        }
+        const int total = __shfl_sync(full, at, 31);
+        at -= count;
+        for (int i = 0; i < count; ++i)
+          am.list[at + i] = (unsigned short)((lane << 8) | (int)((slots >> (8 * i)) & 0xFFu));
+        __syncwarp();
+        // ---- the hits of all rays, 32 at a time
+        for (int base = 0; base < total; base += 32) {
+          const bool on = base + lane < total;
+          const int e = on ? am.list[base + lane] : (32 << 8);
+          const int ray = e >> 8, slot = e & 0xFF;
+          const int before = __shfl_up_sync(full, ray, 1);
+          const unsigned heads = __ballot_sync(full, lane == 0 || ray != before);
+          const int seg = 31 - __clz(heads & (full >> (31 - lane)));
+          const bool tail = on && (lane == 31 || ((heads >> (lane + 1)) & 1u));
+          float* crow = reinterpret_cast<float*>(
+              __shfl_sync(full, reinterpret_cast<unsigned long long>(rows), ray & 31));
+          const int cstride = __shfl_sync(full, rstride, ray & 31);
+          float T0 = -1.0f, S0 = 0.f;
+          float4 q1, q2, q3;  // d, F | g, T | gN, S
+          float4 x0 = make_float4(0.f, 0.f, 0.f, 0.f), x1 = x0;
+          float gD = 0.f;
+          Geom g;
+          float alpha = 0.f, opacity = 0.f, sig = 0.f;
+          uint32_t prim = 0;
+          float3 raw = make_float3(0.f, 0.f, 0.f);
+          if (on) {
+            const unsigned long long key = sm.keys[slot * sm.stride + (ray - lane)];
+            prim = key_prim(key);
+            const float4* tr = p.bvh.tri_prim + 3 * (size_t)prim;
+            const float4 a = __ldg(tr), b = __ldg(tr + 1), c = __ldg(tr + 2);
+            sig = __ldg(p.sigma + prim);
+            opacity = __ldg(p.opac + prim);
+            if (p.cols)
+              raw = make_float3(__ldg(p.cols + 3 * prim), __ldg(p.cols + 3 * prim + 1), __ldg(p.cols + 3 * prim + 2));
+            else if (crow)
+              raw = make_float3(crow[(size_t)(3 * slot) * cstride], crow[(size_t)(3 * slot + 1) * cstride],
+                                crow[(size_t)(3 * slot + 2) * cstride]);
+            const float4 q0 = am.ray[ray];
+            q1 = am.ray[32 + ray];
+            q2 = am.ray[64 + ray];
+            q3 = am.ray[96 + ray];
+            gD = q0.w;
+            T0 = q2.w;
+            S0 = q3.w;
+            if (EXACT) x1 = am.exact[32 + ray];  // gMid, Sd
+            g = shade_geom<MODE>(a, b, c, make_float3(q0.x, q0.y, q0.z), make_float3(q1.x, q1.y, q1.z), key_t(key), sig);
+            alpha = fminf(kAlphaMax, opacity * g.Cx);
+            if (alpha < kAlphaMin) alpha = 0.f;
+          }
+          // transmittance in front of and behind the hit
+          const float prod = seg_product(1.0f - alpha, lane, seg);
+          const float prev = __shfl_up_sync(full, prod, 1);
+          const float T = lane == seg ? T0 : T0 * prev;
+          const float test_T = T * (1.0f - alpha);
+          const unsigned ended = __ballot_sync(full, on && test_T < kTMin);
+          const bool dead = (ended & (full << seg) & (full >> (31 - lane))) != 0u;
+          const bool blend = on && alpha > 0.f && !dead;
+          const float w = blend ? alpha * T : 0.f;
+          float q = 0.f, E = 0.f;
+          if (blend) {
+            if (!p.cols && !crow) {
+              float B[16];
+#pragma unroll
+              for (int i = 0; i < 16; ++i) B[i] = am.basis[16 * ray + i];
+              raw = sh_raw(p.shs, p.M, (int)prim, p.sh_degree, B);
+            }
+            const float c0 = p.cols ? raw.x : fmaxf(raw.x, 0.f), c1 = p.cols ? raw.y : fmaxf(raw.y, 0.f),
+                        c2 = p.cols ? raw.z : fmaxf(raw.z, 0.f);
+            q = q2.x * c0 + q2.y * c1 + q2.z * c2 + gD * g.t + q3.x * g.n.x + q3.y * g.n.y + q3.z * g.n.z;
+            if (EXACT) {
+              x0 = am.exact[ray];  // Df, Wf, distf, gDist
+              const float Cf = x0.y > 0.f ? (x0.z + x0.x * x0.x) / x0.y : 0.f;
+              E = g.t * g.t * x0.y - 2.0f * g.t * x0.x + Cf;
+            }
+          }
+          const float S = S0 + seg_sum(w * q, lane, seg);
+          float Sd = 0.f;
+          if (EXACT) Sd = x1.y + seg_sum(w * E, lane, seg);
+          const unsigned bm = __ballot_sync(full, blend);
+          const int nb = __popc(bm), rank = __popc(bm & ((1u << lane) - 1u));
+          float3 gv[3];
+          if (blend) {
+            const float inv1a = 1.0f / (1.0f - alpha);
+            float dL_dalpha = T * q - (q1.w - S) * inv1a;
+            float dL_dt = gD * w;
+            if (EXACT) {
+              dL_dalpha += x0.w * (T * E - (2.0f * x0.z - Sd) * inv1a);
+              dL_dt += x0.w * 2.0f * w * (g.t * x0.y - x0.x);
+              if (T > 0.5f && test_T <= 0.5f) dL_dt += x1.x;
+            }
+            hit_grads<MODE>(p, prim, g, make_float3(q1.x, q1.y, q1.z), sig, opacity, dL_dalpha, dL_dt,
+                            make_float3(q3.x * w, q3.y * w, q3.z * w), gv);
+            // colour gradients: dRGB/dsh_k = B_k, masked where the colour was clamped at 0
+            const bool m0 = !p.cols && raw.x < 0.f, m1 = !p.cols && raw.y < 0.f, m2 = !p.cols && raw.z < 0.f;
+            const float e0 = m0 ? 0.f : q2.x * w, e1 = m1 ? 0.f : q2.y * w, e2 = m2 ? 0.f : q2.z * w;
+            float4* st = reinterpret_cast<float4*>(am.stage) + 2 * rank;
+            st[0] = make_float4(e0, e1, e2, e0);
+            st[1] = make_float4(e1, __uint_as_float(prim), __int_as_float(ray), 0.f);
+          }
+          __syncwarp();
+          if (sh16) {
+            // two hits of 12 chunks at a time; chunk j holds the products of
+            // coefficients k = 4j / 3 and k + 1, starting at channel j % 3
+            if (lane < 24) {
+              const int j = lane % 12, k = 4 * j / 3, c = j % 3;
+              for (int h = lane / 12; h < nb; h += 2) {
+                const float* st = am.stage + 8 * h;
+                const float* B = am.basis + 16 * __float_as_int(st[6]) + k;
+                const float b0 = B[0], b1 = B[1];
+                const float ea = st[c], eb = st[c + 1], ec = st[c + 2];
+                red_add4(p.d_sh + (size_t)__float_as_uint(st[5]) * 48 + 4 * j, b0 * ea, (c == 2 ? b1 : b0) * eb,
+                         (c == 0 ? b0 : b1) * ec, b1 * ea);
+              }
+            }
+          } else {
+            for (int i = lane; i < nb * row; i += 32) {
+              const int h = i / row, c = i - h * row;
+              const float* st = am.stage + 8 * h;
+              const uint32_t pr = __float_as_uint(st[5]);
+              if (p.cols)
+                red_add(p.d_cols + 3 * (size_t)pr + c, st[c]);
+              else
+                red_add(p.d_sh + (size_t)pr * p.M * 3 + c, am.basis[16 * __float_as_int(st[6]) + c / 3] * st[c % 3]);
+            }
+          }
+          __syncwarp();
+          if (blend) {
+            float* st = am.stage + 9 * rank;
+            st[0] = gv[0].x, st[1] = gv[0].y, st[2] = gv[0].z;
+            st[3] = gv[1].x, st[4] = gv[1].y, st[5] = gv[1].z;
+            st[6] = gv[2].x, st[7] = gv[2].y, st[8] = gv[2].z;
+            am.stage[9 * 32 + rank] = __int_as_float(__ldg(p.cumsum + prim));
+          }
+          __syncwarp();
+          if (lane < 27) {
+            const int c = lane % 9;
+            for (int h = lane / 9; h < nb; h += 3)
+              red_add(p.d_tri + 3 * (size_t)__float_as_int(am.stage[9 * 32 + h]) + c, am.stage[9 * h + c]);
+          }
+          __syncwarp();
+          if (tail) {
+            reinterpret_cast<float*>(am.ray + 64 + ray)[3] = dead ? -1.0f : test_T;
+            reinterpret_cast<float*>(am.ray + 96 + ray)[3] = S;
+            if (EXACT) reinterpret_cast<float*>(am.exact + 32 + ray)[1] = Sd;
+          }
+          __syncwarp();
+        }
+        if (marching || active) {
+          if (reinterpret_cast<const float*>(am.ray + 64 + lane)[3] < 0.f) marching = active = false;
+        }
+      }
+    }
+    __syncwarp();
+  }
+  if (lane == 0 && replays != 0u) atomicAdd(p.stats + kStatReplays, (unsigned long long)replays);
 }
 
 // ---------------------------------------------------------------- secondary rays
@@ -3172,6 +3545,8 @@ cudaError_t opt_in_kernels() {
   opt_in((const void*)k_collect<CFG>, smem_bytes_for<CFG>());
   opt_in((const void*)k_forward<CFG, MODE>, smem_bytes_for<CFG>() + extra);
   opt_in((const void*)k_backward<CFG, MODE>, smem_bytes_for<CFG>());
+  if constexpr (TraversalCfg<CFG>::packets)
+    opt_in((const void*)k_adjoint<TraversalCfg<CFG>::K, MODE>, adjoint_smem<TraversalCfg<CFG>::K, MODE>());
   return e;
 }
 
@@ -3200,6 +3575,7 @@ static_assert(smem_bytes_for<kCfgPackets32, true>() + kExactSmemBytes <= 48 * 10
 // Grid of a replay-only build: the traversing build's grid (SMs x its blocks
 // per SM) at the replay build's blocks per SM.
 inline int replay_grid(int grid) { return grid / kMinBlocks * kReplayBlocks; }
+inline int adjoint_grid(int grid) { return grid / kMinBlocks * kAdjointBlocks; }
 
 template <int MODE>
 cudaError_t launch_forward_t(const TraceParams& p, int grid, cudaStream_t s) {
@@ -3223,9 +3599,9 @@ template <int MODE>
 cudaError_t launch_backward_t(const TraceParams& p, int grid, cudaStream_t s) {
   if (p.bwd_pair) {
     if (p.cfg == kCfgPackets16)
-      k_backward<kCfgPackets16, MODE, true><<<replay_grid(grid), kTraceThreads, smem_bytes_for<kCfgPackets16, true>(), s>>>(p);
+      k_adjoint<16, MODE><<<adjoint_grid(grid), kTraceThreads, adjoint_smem<16, MODE>(), s>>>(p);
     else
-      k_backward<kCfgPackets32, MODE, true><<<replay_grid(grid), kTraceThreads, smem_bytes_for<kCfgPackets32, true>(), s>>>(p);
+      k_adjoint<32, MODE><<<adjoint_grid(grid), kTraceThreads, adjoint_smem<32, MODE>(), s>>>(p);
   }
   switch (p.cfg) {
     case kCfgPackets16: k_backward<kCfgPackets16, MODE><<<grid, kTraceThreads, smem_bytes_for<kCfgPackets16>(), s>>>(p); break;
