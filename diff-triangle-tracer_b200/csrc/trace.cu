@@ -1283,18 +1283,18 @@ __device__ __forceinline__ bool cache_colors_on(const TraceParams& p) {
   if (!p.cache_colors || p.cols) return false;
   return p.cache_mode != kCacheRead || (cache_header_ptr(p)->k & kCacheColorsFlag) != 0u;
 }
-// Colour rows of the main-part entry of ray g or of pool entry e (row 3i + c
-// holds channel c of slot i; `stride` floats between rows). Both counts fit
-// an int: every entry takes over 400 bytes of the buffer.
+// Colours of the main-part entry of ray g or of pool entry e (slot i's three
+// channels at i * stride). Three times either count fits an int: every entry
+// takes over 400 bytes of the buffer.
 template <int K>
 __device__ __forceinline__ float* cache_color_rows(const TraceParams& p, bool main_part, long long g, uint32_t e,
                                                    int& stride) {
   if (main_part) {
-    stride = (int)p.cache_rays;
-    return p.cache_colors + g;
+    stride = 3 * (int)p.cache_rays;
+    return p.cache_colors + 3 * (size_t)g;
   }
-  stride = (int)p.cache_pool_cap;
-  return p.cache_colors + (size_t)3 * K * p.cache_rays + e;
+  stride = 3 * (int)p.cache_pool_cap;
+  return p.cache_colors + (size_t)3 * K * p.cache_rays + 3 * (size_t)e;
 }
 
 // Shaders that use the colour rows take them and the hit's slot; the others
@@ -1722,8 +1722,8 @@ struct FwdShader {
   // per-thread shared-memory slot (kExactSlots words, stride blockDim.x), so
   // the traversal between two shading passes does not carry them in registers
   float* xs = nullptr;
-  // colour rows of the current query's hit-cache entry (raw colour of the
-  // hit in slot i at rows 3i..3i+2, `cstride` floats apart), or nullptr
+  // colours of the current query's hit-cache entry (raw colour of the hit in
+  // slot i at i * cstride), or nullptr
   float* crow = nullptr;
   int cstride = 0;
   unsigned n_rays = 0, n_eval = 0, n_blend = 0;
@@ -1821,9 +1821,9 @@ struct FwdShader {
       const float3 raw = sh_raw(p.shs, p.M, (int)prim, p.sh_degree, B);
       c = make_float3(fmaxf(raw.x, 0.f), fmaxf(raw.y, 0.f), fmaxf(raw.z, 0.f));
       if (crow && slot >= 0) {  // for the adjoint, which then reads it instead of the SH
-        crow[(size_t)(3 * slot) * cstride] = raw.x;
-        crow[(size_t)(3 * slot + 1) * cstride] = raw.y;
-        crow[(size_t)(3 * slot + 2) * cstride] = raw.z;
+        crow[(size_t)slot * cstride] = raw.x;
+        crow[(size_t)slot * cstride + 1] = raw.y;
+        crow[(size_t)slot * cstride + 2] = raw.z;
       }
     }
     C0 += c.x * w;
@@ -2342,8 +2342,8 @@ struct BwdShader {
     } else {
       sh_basis(unit(d), p.sh_degree, B);
       if (crow && slot >= 0)
-        raw = make_float3(crow[(size_t)(3 * slot) * cstride], crow[(size_t)(3 * slot + 1) * cstride],
-                          crow[(size_t)(3 * slot + 2) * cstride]);
+        raw = make_float3(crow[(size_t)slot * cstride], crow[(size_t)slot * cstride + 1],
+                          crow[(size_t)slot * cstride + 2]);
       else
         raw = sh_raw(p.shs, p.M, (int)prim, p.sh_degree, B);
     }
@@ -2593,8 +2593,8 @@ __global__ void __launch_bounds__(kTraceThreads, kAdjointBlocks) k_adjoint(const
             if (p.cols)
               raw = make_float3(__ldg(p.cols + 3 * prim), __ldg(p.cols + 3 * prim + 1), __ldg(p.cols + 3 * prim + 2));
             else if (crow)
-              raw = make_float3(crow[(size_t)(3 * slot) * cstride], crow[(size_t)(3 * slot + 1) * cstride],
-                                crow[(size_t)(3 * slot + 2) * cstride]);
+              raw = make_float3(crow[(size_t)slot * cstride], crow[(size_t)slot * cstride + 1],
+                                crow[(size_t)slot * cstride + 2]);
             const float4 q0 = am.ray[ray];
             q1 = am.ray[32 + ray];
             q2 = am.ray[64 + ray];

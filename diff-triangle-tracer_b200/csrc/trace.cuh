@@ -52,11 +52,13 @@ __host__ __device__ inline size_t hit_cache_main_bytes(int k, long long rays) {
   return sizeof(HitCacheHeader) + (size_t)(k + 1) * 8 * (size_t)rays;
 }
 // The plain forward / adjoint's cache also holds each stored query's hit
-// colours after the pool: per entry (main part, then pool) 3k float rows,
-// the raw (unclamped) colour of the hit in slot i in rows 3i, 3i + 1, 3i + 2.
-// The shading pass writes the colour of every hit it blends and the adjoint
-// reads it instead of evaluating the hit's SH again. Header k carries
-// kCacheColorsFlag when the colours were written.
+// colours after the pool: per part (main, then pool) k rows of three floats an
+// entry, the raw (unclamped) colour of the hit in slot i in row i. The shading
+// pass writes the colour of every hit it blends and the adjoint reads it
+// instead of evaluating the hit's SH again; the three channels are neighbours,
+// so a lane that takes one hit touches one or two sectors (a row a channel:
+// adjoint of 1M triangles, 2.56M rays 3.26 instead of 3.16 ms). Header k
+// carries kCacheColorsFlag when the colours were written.
 constexpr uint32_t kCacheColorsFlag = 0x10000u;
 __host__ __device__ inline size_t hit_cache_color_bytes(int k, long long entries) {
   return (size_t)12 * k * (size_t)entries;
