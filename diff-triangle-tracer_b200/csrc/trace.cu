@@ -373,6 +373,56 @@ __device__ __forceinline__ void kb_sort(unsigned long long* kb, int stride, int 
   }
 }
 
+// A lane's (triangle, ray) pair, `ray` a lane of the warp: the watertight test
+// with that lane's ray, a hit appended to that lane's buffer. When a buffer has
+// no room, all are sorted and cut back to their K nearest, which bound their
+// rays' tmax, and what did not fit tries again if still near enough: returns
+// true then. `hits`: keys in each lane's buffer; kb_n: how many of this lane's
+// are in order.
+template <int K>
+__device__ __forceinline__ bool test_pairs(const RayW& r, unsigned long long key_min, float& tmax, int& kb_n,
+                                           unsigned long long* kb, int kstride, int* hits, bool have, int ray, float4 a,
+                                           float4 b, float4 c) {
+  const unsigned full = 0xFFFFFFFFu;
+  const int lane = threadIdx.x & 31;
+  RayW q;
+  q.ox = __shfl_sync(full, r.ox, ray), q.oy = __shfl_sync(full, r.oy, ray), q.oz = __shfl_sync(full, r.oz, ray);
+  q.Sx = __shfl_sync(full, r.Sx, ray), q.Sy = __shfl_sync(full, r.Sy, ray), q.Sz = __shfl_sync(full, r.Sz, ray);
+  q.perm = __shfl_sync(full, r.perm, ray);
+  const unsigned long long lo = __shfl_sync(full, key_min, ray);
+  const float far = __shfl_sync(full, tmax, ray);
+  unsigned long long key = kEmptyKey;
+  if (have) {
+    float t;
+    if (isect_tri_p(q, PermRt(q.perm), a, b, c, t) && t >= 0.f && t <= far) {
+      key = hit_key(t, (uint32_t)__float_as_int(a.w));
+      if (key < lo) key = kEmptyKey;
+    }
+  }
+  bool cut = false;
+  while (__any_sync(full, key != kEmptyKey)) {
+    if (key != kEmptyKey) {
+      const int slot = atomicAdd(hits + ray, 1);
+      if (slot < K + kSpare) {
+        kb[slot * kstride + (ray - lane)] = key;
+        key = kEmptyKey;
+      }
+    }
+    if (!__any_sync(full, key != kEmptyKey)) break;
+    cut = true;
+    __syncwarp();
+    const int n = min(hits[lane], K + kSpare);
+    kb_sort(kb, kstride, kb_n, n);
+    kb_n = min(n, K);
+    hits[lane] = kb_n;
+    if (kb_n == K) tmax = fminf(tmax, key_t(kb[(K - 1) * kstride]));
+    __syncwarp();
+    const float nearer = __shfl_sync(full, tmax, ray);
+    if (key != kEmptyKey && key_t(key) > nearer) key = kEmptyKey;
+  }
+  return cut;
+}
+
 // The rays (bits, ray i of the packet in bit i) that may hit a triangle, given
 // as its vertices relative to the common origin in (u, v, z'): all three edge
 // planes through the origin have the ray on the inner side, up to 2^-18 of
@@ -575,42 +625,8 @@ __device__ __forceinline__ void packet_query(const BvhView& bvh, const RayW& r, 
             c.x = __shfl_sync(full, C.x, tri), c.y = __shfl_sync(full, C.y, tri), c.z = __shfl_sync(full, C.z, tri);
             a.w = __shfl_sync(full, A.w, tri);
             b.w = c.w = 0.f;
-            const unsigned long long lo = __shfl_sync(full, key_min, ray);
-            RayW q;
-            q.ox = __shfl_sync(full, r.ox, ray), q.oy = __shfl_sync(full, r.oy, ray), q.oz = __shfl_sync(full, r.oz, ray);
-            q.Sx = __shfl_sync(full, r.Sx, ray), q.Sy = __shfl_sync(full, r.Sy, ray), q.Sz = __shfl_sync(full, r.Sz, ray);
-            q.perm = __shfl_sync(full, r.perm, ray);
-            const float far = __shfl_sync(full, tmax, ray);
-            unsigned long long key = kEmptyKey;
-            if (have) {
-              float t;
-              if (isect_tri_p(q, PermRt(q.perm), a, b, c, t) && t >= 0.f && t <= far) {
-                key = hit_key(t, (uint32_t)__float_as_int(a.w));
-                if (key < lo) key = kEmptyKey;
-              }
-            }
-            while (__any_sync(full, key != kEmptyKey)) {
-              if (key != kEmptyKey) {
-                const int slot = atomicAdd(ws.hits + ray, 1);
-                if (slot < K + kSpare) {
-                  kb[slot * kstride + (ray - lane)] = key;
-                  key = kEmptyKey;
-                }
-              }
-              if (!__any_sync(full, key != kEmptyKey)) break;
-              // A buffer has no room: all are sorted and cut back to their K
-              // nearest, and what did not fit tries again if still near enough
-              __syncwarp();
-              const int n = min(ws.hits[lane], K + kSpare);
-              kb_sort(kb, kstride, kb_n, n);
-              kb_n = min(n, K);
-              ws.hits[lane] = kb_n;
-              if (kb_n == K) tmax = fminf(tmax, key_t(kb[(K - 1) * kstride]));
+            if (test_pairs<K>(r, key_min, tmax, kb_n, kb, kstride, ws.hits, have, ray, a, b, c))
               zcur = fminf(z1, warp_max(in ? fmaf(tmax, dk, oz) : -INFINITY) + pad);
-              __syncwarp();
-              const float nearer = __shfl_sync(full, tmax, ray);
-              if (key != kEmptyKey && key_t(key) > nearer) key = kEmptyKey;
-            }
           }
           __syncwarp();
         }
@@ -724,6 +740,159 @@ __device__ __forceinline__ void packet_query(const BvhView& bvh, const RayW& r, 
   const int n = min(ws.hits[lane], K + kSpare);
   kb_sort(kb, kstride, kb_n, n);
   for (int i = n; i < K; ++i) kb[i * kstride] = kEmptyKey;
+}
+
+// ---------------------------------------------------------------- pairs
+// Queries of unrelated rays, a warp's worth at a time. Traversed a ray a lane,
+// such rays leave most lanes idle (7 of 32 active on the spawned levels of the
+// benchmark's secondary rays): they differ in when they are at a node, at a
+// leaf, inserting a hit or done. Here the warp keeps one stack of (node, ray)
+// pairs; a lane takes any pair, tests its ray against the node's 8 children and
+// adds the entered ones, triangles to a queue of (triangle, ray) pairs that are
+// tested 32 at a time.
+//
+// Traversal of the spawned rays of 500k triangles, 2 views of 800^2, two
+// bounces (1.87M rays, 99 node visits and 58 triangle tests each): 15.2 ms a
+// ray a lane, 9.9 with pairs added slot by slot, 7.9 with each lane's triangles
+// in one run (26 lanes at work in a node step, 32 in a triangle step). It
+// issues on half of the cycles, the rest waits on arithmetic and on L1, whose
+// bandwidth is half used by the node loads. A frustum around 32 of these rays,
+// or one around each ray for the whole warp, takes 38-41 ms.
+constexpr int kPairStack = 512;    // (node << 5 | ray); nodes and triangles are below 2^27
+constexpr int kPairReserve = 200;  // kept free for pairs taken one at a time (a depth-first walk adds 7 a level)
+constexpr int kPairQueue = 512;    // (triangle << 5 | ray), ring
+struct PairMem {
+  uint32_t* stack;
+  uint32_t* queue;
+  int* hits;  // [32] keys in each lane's buffer
+  int* drop;  // [32] float bits of the nearest dropped entry distance
+};
+constexpr size_t kPairBytes = (size_t)(kPairStack + kPairQueue + 64) * 4;
+template <int K>
+constexpr size_t pair_smem() {
+  return (size_t)kTraceThreads * (K + kSpare) * 8 + (size_t)(kTraceThreads / 32) * kPairBytes;
+}
+
+template <int K>
+__device__ __forceinline__ void pair_query(const BvhView& bvh, const RayW& r, bool want, unsigned long long key_min,
+                                           float t_hi, unsigned long long* kb, int kstride, PairMem pm, float& t_drop,
+                                           int* status, Counters& cnt, int count_work) {
+  const unsigned full = 0xFFFFFFFFu;
+  const int lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1u;
+  float tmax = t_hi;
+  const float t_lo = key_t(key_min);
+  int kb_n = 0;
+  const unsigned act = __ballot_sync(full, want && bvh.has_root);
+  if (want) ++cnt.queries;
+  pm.hits[lane] = 0;
+  pm.drop[lane] = __float_as_int(INFINITY);
+  if ((act >> lane) & 1u) pm.stack[__popc(act & lt)] = (uint32_t)lane;  // the root, with every ray
+  int sp = __popc(act), qh = 0, qn = 0;
+  __syncwarp();
+  for (int steps = 0; sp + qn > 0; ++steps) {
+    if (steps > kMaxSteps) {
+      if (lane == 0) atomicOr(status, kStatusTimeout);
+      break;
+    }
+    if (qn >= 32 || sp == 0) {
+      const int n = min(qn, 32);
+      const uint32_t e = lane < n ? pm.queue[(qh + lane) & (kPairQueue - 1)] : 0u;
+      qh += n;
+      qn -= n;
+      const float4* tr = bvh.tris + 3 * (size_t)(e >> 5);
+      const float4 a = __ldg(tr), b = __ldg(tr + 1), c = __ldg(tr + 2);
+      if (count_work && lane < n) ++cnt.tris;
+      test_pairs<K>(r, key_min, tmax, kb_n, kb, kstride, pm.hits, lane < n, (int)(e & 31u), a, b, c);
+      __syncwarp();
+      continue;
+    }
+    int m = min(min(sp, 32), max((kPairStack - kPairReserve - sp) / 7, 1));
+    const uint32_t e = lane < m ? pm.stack[sp - 1 - lane] : 0u;
+    const int ray = (int)(e & 31u);
+    RayW q;
+    q.ix = __shfl_sync(full, r.ix, ray), q.iy = __shfl_sync(full, r.iy, ray), q.iz = __shfl_sync(full, r.iz, ray);
+    q.oix = __shfl_sync(full, r.oix, ray), q.oiy = __shfl_sync(full, r.oiy, ray), q.oiz = __shfl_sync(full, r.oiz, ray);
+    const float lo = __shfl_sync(full, t_lo, ray), hi = __shfl_sync(full, tmax, ray);
+    const bool ok = TT_IN_BOUNDS(status, (e >> 5) < (uint32_t)bvh.wide_cap);
+    const float4* nd = bvh.nodes + (size_t)(ok ? e >> 5 : 0u) * kNodeF4;
+    const int nx = q.ix >= 0.f ? 0 : 2, ny = q.iy >= 0.f ? 4 : 6, nz = q.iz >= 0.f ? 8 : 10;
+    float tn[8], tf[8];
+    const float4 r0 = __ldg(nd + 12), r1 = __ldg(nd + 13);
+    slab8(nd, nx, ny, nz, q, lo, hi, tn, tf);
+    const uint32_t cref[8] = {__float_as_uint(r0.x), __float_as_uint(r0.y), __float_as_uint(r0.z),
+                              __float_as_uint(r0.w), __float_as_uint(r1.x), __float_as_uint(r1.y),
+                              __float_as_uint(r1.z), __float_as_uint(r1.w)};
+    int tris = 0;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) tris += tn[c] <= tf[c] && ref_is_leaf(cref[c]) ? (int)leaf_count(cref[c]) : 0;
+    // triangles: each lane's in one run; fewer pairs if they would not fit
+    int at;
+    for (;; m >>= 1) {
+      if (lane >= m) tris = 0;
+      at = tris;
+#pragma unroll
+      for (int i = 1; i < 32; i <<= 1) {
+        const int u = __shfl_up_sync(full, at, i);
+        if (lane >= i) at += u;
+      }
+      const int total = __shfl_sync(full, at, 31);
+      at += qh + qn - tris;
+      if (total <= kPairQueue - qn || m == 1) {
+        qn += total;
+        break;
+      }
+    }
+    const bool on = lane < m;
+    if (count_work && on) ++cnt.nodes;
+    __syncwarp();
+    sp -= m;
+    unsigned inner[8];
+    int more = 0;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const bool h = on && tn[c] <= tf[c], leaf = ref_is_leaf(cref[c]);
+      inner[c] = __ballot_sync(full, h && !leaf);
+      more += __popc(inner[c]);
+      if (h && leaf) {
+        const uint32_t first = leaf_first(cref[c]), n = leaf_count(cref[c]);
+        const uint32_t f = ((TT_IN_BOUNDS(status, first + n <= (uint32_t)bvh.P) ? first : 0u) << 5) | (uint32_t)ray;
+        pm.queue[at & (kPairQueue - 1)] = f;
+        if (n > 1u) pm.queue[(at + 1) & (kPairQueue - 1)] = f + 32u;
+        if (n > 2u) pm.queue[(at + 2) & (kPairQueue - 1)] = f + 64u;
+        at += (int)n;
+      }
+    }
+    // interior children: slot by slot, so that rays entering the same child lie
+    // side by side and share its loads
+    if (sp + more <= kPairStack) {
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        if ((inner[c] >> lane) & 1u) pm.stack[sp + __popc(inner[c] & lt)] = (cref[c] << 5) | (uint32_t)ray;
+        sp += __popc(inner[c]);
+      }
+    } else {
+      // no room: the rays only trust keys nearer than what they had to drop
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        if ((inner[c] >> lane) & 1u) {
+          const int to = sp + __popc(inner[c] & lt);
+          if (to < kPairStack)
+            pm.stack[to] = (cref[c] << 5) | (uint32_t)ray;
+          else
+            atomicMin(pm.drop + ray, __float_as_int(tn[c]));
+        }
+        sp = min(sp + __popc(inner[c]), kPairStack);
+      }
+    }
+    __syncwarp();
+  }
+  __syncwarp();
+  const int n = min(pm.hits[lane], K + kSpare);
+  kb_sort(kb, kstride, kb_n, n);
+  for (int i = n; i < K; ++i) kb[i * kstride] = kEmptyKey;
+  t_drop = __int_as_float(pm.drop[lane]);
+  __syncwarp();
 }
 
 // ---------------------------------------------------------------- shading
@@ -1488,6 +1657,15 @@ __device__ __forceinline__ void drive(const TraceParams& p, const Smem& sm, Shad
       }
     }
   }
+}
+
+__device__ __forceinline__ PairMem pair_mem(unsigned char* base) {
+  PairMem pm;
+  pm.stack = reinterpret_cast<uint32_t*>(base + (size_t)(threadIdx.x >> 5) * kPairBytes);
+  pm.queue = pm.stack + kPairStack;
+  pm.hits = reinterpret_cast<int*>(pm.queue + kPairQueue);
+  pm.drop = pm.hits + 32;
+  return pm;
 }
 
 // Packet driver: a warp takes an 8x4-pixel tile, then runs rounds of one
@@ -2731,10 +2909,11 @@ __global__ void __launch_bounds__(kTraceThreads, kAdjointBlocks) k_adjoint(const
 // colour from the children's resolved radiance.
 
 // Per-lane persistent driver over `total` queue items (item order = record
-// order); lanes refill as their rays finish.
+// order); lanes refill as their rays finish. With SD = 0 the queries go through
+// the warp's pair stack `pm` instead of a stack a lane.
 template <int SD, class Shader>
 __device__ __forceinline__ void drive_items(const TraceParams& p, const Smem& sm, Shader& sh, Counters& cnt,
-                                            int total) {
+                                            int total, PairMem pm = PairMem{}) {
   constexpr int K = kChunk;
   const unsigned full = 0xFFFFFFFFu;
   const int lane = threadIdx.x & 31;
@@ -2768,6 +2947,9 @@ __device__ __forceinline__ void drive_items(const TraceParams& p, const Smem& sm
       continue;
     }
     float t_drop = INFINITY;
+    if constexpr (SD == 0)  // (no queries to replay where pairs are used)
+      pair_query<K>(p.bvh, make_ray(o, d), have, cur.key_min, cur.t_hi, sm.keys, sm.stride, pm, t_drop, p.status, cnt,
+                    p.count_work);
     if (have) {
       // Hit cache: a level-0 ray (record = pixel) keeps its first query in
       // the main part; a deeper ray starts its chain in the pool, linked from
@@ -2782,8 +2964,10 @@ __device__ __forceinline__ void drive_items(const TraceParams& p, const Smem& sm
         ++cnt.replays;
       } else {
         next = kNoEntry;
-        const RayW r = make_ray(o, d);
-        query<SD>(p.bvh, r, cur.key_min, cur.t_hi, sm.keys, sm.stride, sm.st, t_drop, p.status, cnt, p.count_work);
+        if constexpr (SD != 0) {
+          const RayW r = make_ray(o, d);
+          query<SD>(p.bvh, r, cur.key_min, cur.t_hi, sm.keys, sm.stride, sm.st, t_drop, p.status, cnt, p.count_work);
+        }
         if (p.cache_mode == kCacheWrite || p.cache_mode == kCacheFill) {
           if (main_part) {
             link = cache_put_first<K>(p, sh.ridx, sm, t_drop);
@@ -3124,17 +3308,14 @@ __global__ void __launch_bounds__(kTraceThreads, kSecBlocks) k_sec_trace(const _
 // the same order, with a shader that shades and spawns nothing, storing every
 // query in the ray tree's hit cache (the chain starts at the ray's record);
 // k_sec_trace then replays them in fill mode. Like k_collect for primary
-// rays: without the shading and spawning code the pass needs fewer
-// registers, and with a shorter shared-memory stack per lane (continued in
-// local memory) more blocks fit an SM.
-#ifndef TT_SEC_COLLECT_STACK
-#define TT_SEC_COLLECT_STACK 16
-#endif
+// rays, it needs fewer registers without the shading and spawning code; its
+// rays are traced as pairs. 5 blocks per SM (96 registers): 7.9 ms on the
+// workload above, 8.0 at 4.
 #ifndef TT_SEC_COLLECT_BLOCKS
-#define TT_SEC_COLLECT_BLOCKS 6
+#define TT_SEC_COLLECT_BLOCKS 5
 #endif
-constexpr int kSecCollectStack = TT_SEC_COLLECT_STACK, kSecCollectBlocks = TT_SEC_COLLECT_BLOCKS;
-constexpr size_t sec_collect_smem() { return (size_t)kTraceThreads * (kSecCollectStack * 8 + kChunk * 8); }
+constexpr int kSecCollectBlocks = TT_SEC_COLLECT_BLOCKS;
+constexpr size_t sec_collect_smem() { return pair_smem<kChunk>(); }
 
 struct SecMarchShader {
   static constexpr bool kStopsAtClip = true;
@@ -3156,7 +3337,9 @@ struct SecMarchShader {
 __global__ void __launch_bounds__(kTraceThreads, kSecCollectBlocks) k_sec_collect(const __grid_constant__ TraceParams p) {
   Counters cnt;
   SecMarchShader sh(p);
-  drive_items<kSecCollectStack>(p, thread_smem<kSecCollectStack>(), sh, cnt, sec_level_size(p, p.sec.level));
+  unsigned char* rest;
+  const Smem sm = packet_smem<kChunk>(rest);
+  drive_items<0>(p, sm, sh, cnt, sec_level_size(p, p.sec.level), pair_mem(rest));
   cnt.queries = 0;  // counted by the shading pass (k_sec_trace), like k_collect
   add_stats(p.stats, 0u, 0u, 0u, cnt);
 }
