@@ -45,8 +45,16 @@ void DevBuf::release() {
 namespace {
 
 constexpr int kBlock = 256;
-constexpr int kSortItems = 16;
-constexpr int kSortTile = kBlock * kSortItems;
+// Keys a thread sorts: 16, or 8 or 4 while the tiles still number at most
+// kSortTiles, the most one block scans. A pass walks its tile in rounds of 256
+// keys with block barriers, so a small sort takes as long as a tile does
+// (20k pairs: 23 us a pass at 16 keys, 12 at 4; 61k pairs: 21 at 16, 17 at 8).
+constexpr int kSortTiles = 32;
+int sort_items(size_t n) { return n <= (size_t)kSortTiles * kBlock * 4 ? 4 : (n <= (size_t)kSortTiles * kBlock * 8 ? 8 : 16); }
+size_t sort_tiles(size_t n) {
+  const size_t tile = (size_t)kBlock * sort_items(n);
+  return (n + tile - 1) / tile;
+}
 
 struct alignas(16) BinNode {
   float4 lo, hi;
@@ -146,14 +154,15 @@ __global__ void k_morton(const float4* __restrict__ cen, const int* __restrict__
 }
 
 // ------------------------------------------------------------- radix sort
+template <int kItems>
 __global__ void k_sort_hist(const uint32_t* __restrict__ keys, int n, int shift, uint32_t* __restrict__ hist,
                             int tiles) {
   __shared__ uint32_t h[256];
   h[threadIdx.x] = 0;
   __syncthreads();
-  const int base = blockIdx.x * kSortTile;
+  const int base = blockIdx.x * (kBlock * kItems);
 #pragma unroll 4
-  for (int i = 0; i < kSortItems; ++i) {
+  for (int i = 0; i < kItems; ++i) {
     const int idx = base + i * kBlock + threadIdx.x;
     if (idx < n) atomicAdd(&h[(keys[idx] >> shift) & 255u], 1u);
   }
@@ -264,9 +273,10 @@ void scan_hist(uint32_t* hist, int tiles, cudaStream_t s) {
   k_scan_add<<<chunks, kScanThreads, 0, s>>>(hist, n, sums);
 }
 
-// Stable scatter of one tile: keys are visited in index order (16 rounds of
+// Stable scatter of one tile: keys are visited in index order (kItems rounds of
 // 256), ranked within each warp with __match_any_sync and across warps with a
 // per-digit prefix in shared memory.
+template <int kItems>
 __global__ void k_sort_scatter(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin,
                                uint32_t* __restrict__ kout, uint32_t* __restrict__ vout, int n, int shift,
                                const uint32_t* __restrict__ offsets, int tiles) {
@@ -275,8 +285,8 @@ __global__ void k_sort_scatter(const uint32_t* __restrict__ kin, const uint32_t*
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   run[threadIdx.x] = offsets[threadIdx.x * tiles + blockIdx.x];
   const unsigned lt = (1u << lane) - 1u;
-  const int base = blockIdx.x * kSortTile;
-  for (int it = 0; it < kSortItems; ++it) {
+  const int base = blockIdx.x * (kBlock * kItems);
+  for (int it = 0; it < kItems; ++it) {
     const int idx = base + it * kBlock + threadIdx.x;
     const bool valid = idx < n;
     const uint32_t k = valid ? kin[idx] : 0u;
@@ -306,6 +316,24 @@ __global__ void k_sort_scatter(const uint32_t* __restrict__ kin, const uint32_t*
       vout[pos] = v;
     }
     __syncthreads();
+  }
+}
+
+// One pass over n pairs by the 8 bits at `shift`.
+template <int kItems>
+void sort_pass_t(const uint32_t* ka, const uint32_t* va, uint32_t* kb, uint32_t* vb, uint32_t* hist, int n, int shift,
+                 cudaStream_t s) {
+  const int tiles = (int)sort_tiles((size_t)n);
+  k_sort_hist<kItems><<<tiles, kBlock, 0, s>>>(ka, n, shift, hist, tiles);
+  scan_hist(hist, tiles, s);
+  k_sort_scatter<kItems><<<tiles, kBlock, 0, s>>>(ka, va, kb, vb, n, shift, hist, tiles);
+}
+void sort_pass(const uint32_t* ka, const uint32_t* va, uint32_t* kb, uint32_t* vb, uint32_t* hist, int n, int shift,
+               cudaStream_t s) {
+  switch (sort_items((size_t)n)) {
+    case 4: sort_pass_t<4>(ka, va, kb, vb, hist, n, shift, s); break;
+    case 8: sort_pass_t<8>(ka, va, kb, vb, hist, n, shift, s); break;
+    default: sort_pass_t<16>(ka, va, kb, vb, hist, n, shift, s); break;
   }
 }
 
@@ -364,34 +392,126 @@ __device__ __forceinline__ void tri_box(const float4* __restrict__ tri, int pos,
   hi = make_float4(fmaxf(a.x, fmaxf(b.x, c.x)), fmaxf(a.y, fmaxf(b.y, c.y)), fmaxf(a.z, fmaxf(b.z, c.z)), 0.f);
 }
 
+// Box of a binary subtree that another block may just have written.
 __device__ __forceinline__ void child_box(const BinNode* bn, const float4* tri, int ref, float4& lo, float4& hi) {
   if (ref >= 0) {
     lo = __ldcg(&bn[ref].lo);
     hi = __ldcg(&bn[ref].hi);
   } else {
-    tri_box(tri, ~ref, lo, hi);
+    const float4* t = tri + 3 * (size_t)~ref;
+    const float4 a = __ldcg(t), b = __ldcg(t + 1), c = __ldcg(t + 2);
+    lo = make_float4(fminf(a.x, fminf(b.x, c.x)), fminf(a.y, fminf(b.y, c.y)), fminf(a.z, fminf(b.z, c.z)), 0.f);
+    hi = make_float4(fmaxf(a.x, fmaxf(b.x, c.x)), fmaxf(a.y, fmaxf(b.y, c.y)), fmaxf(a.z, fmaxf(b.z, c.z)), 0.f);
   }
 }
 
-__global__ void k_bottom_up(const float4* __restrict__ tri, int P, BinNode* bn, const int* __restrict__ bparent,
-                            const int* __restrict__ lparent, int* flags) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P || P < 2) return;
-  int node = lparent[p];
-  while (node >= 0) {
-    __threadfence();
-    if (atomicAdd(&flags[node], 1) == 0) return;
-    __threadfence();
-    float4 l0, h0, l1, h1;
-    const int left = __ldcg(&bn[node].left), right = __ldcg(&bn[node].right);
-    child_box(bn, tri, left, l0, h0);
-    child_box(bn, tri, right, l1, h1);
-    const float4 lo = make_float4(fminf(l0.x, l1.x), fminf(l0.y, l1.y), fminf(l0.z, l1.z), 0.f);
-    const float4 hi = make_float4(fmaxf(h0.x, h1.x), fmaxf(h0.y, h1.y), fmaxf(h0.z, h1.z), 0.f);
+// Boxes of the binary tree, bottom up: a thread starts at its leaf with the
+// box in registers and goes on at each node as the second of its two children
+// to arrive. A level costs a round trip to L2 for the node, a fence and an
+// atomic, and the chain of levels is what this pass takes, so a block keeps the
+// nodes over its own kClimb leaves to itself: there the first child leaves its box
+// in shared memory. (Karras numbers a node by one end of its range, so those
+// nodes index the block's slots.) Only the levels above go through global
+// flags, which the second arrival clears for the next refit.
+constexpr int kClimb = 256;  // leaves a block
+struct ClimbMem {
+  float box[2][kClimb][6];
+  int seen[kClimb];
+};
+// The arrival at a node: releases what this thread wrote and acquires what the
+// other child's did (cheaper than a fence on both sides).
+__device__ __forceinline__ int arrive(int* flag) {
+  int seen;
+  asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(seen) : "l"(flag) : "memory");
+  return seen;
+}
+__device__ __forceinline__ void climb(ClimbMem& sm, int leaf, int b0, float4 lo, float4 hi, const float4* tri,
+                                      BinNode* bn, const int* __restrict__ bparent, const int* __restrict__ lparent,
+                                      int* flags) {
+  int child = ~leaf, node = lparent[leaf];
+  int up = bparent[node];
+  int4 t = *reinterpret_cast<const int4*>(&bn[node].left);  // left, right, first, last
+  for (;;) {
+    // the parent's links, under way while this node is settled
+    const int up2 = up >= 0 ? bparent[up] : -1;
+    const int4 t2 = up >= 0 ? *reinterpret_cast<const int4*>(&bn[up].left) : t;
+    const int side = t.x == child ? 0 : 1;
+    float4 l1, h1;
+    if (t.z >= b0 && t.w < b0 + kClimb) {
+      const int k = node - b0;
+      float* mine = sm.box[side][k];
+      mine[0] = lo.x, mine[1] = lo.y, mine[2] = lo.z, mine[3] = hi.x, mine[4] = hi.y, mine[5] = hi.z;
+      __threadfence_block();
+      if (atomicAdd(&sm.seen[k], 1) == 0) return;
+      __threadfence_block();
+      const volatile float* o = sm.box[side ^ 1][k];
+      l1 = make_float4(o[0], o[1], o[2], 0.f);
+      h1 = make_float4(o[3], o[4], o[5], 0.f);
+    } else {
+      if (arrive(&flags[node]) == 0) return;
+      flags[node] = 0;
+      child_box(bn, tri, side == 0 ? t.y : t.x, l1, h1);
+    }
+    lo = make_float4(fminf(lo.x, l1.x), fminf(lo.y, l1.y), fminf(lo.z, l1.z), 0.f);
+    hi = make_float4(fmaxf(hi.x, h1.x), fmaxf(hi.y, h1.y), fmaxf(hi.z, h1.z), 0.f);
     __stcg(&bn[node].lo, lo);
     __stcg(&bn[node].hi, hi);
-    node = bparent[node];
+    if (up < 0) return;
+    child = node;
+    node = up;
+    up = up2;
+    t = t2;
   }
+}
+
+// (flags zero at launch)
+__global__ void __launch_bounds__(kClimb) k_bottom_up(const float4* __restrict__ tri, int P, BinNode* bn,
+                                                      const int* __restrict__ bparent, const int* __restrict__ lparent,
+                                                      int* flags) {
+  __shared__ ClimbMem sm;
+  const int b0 = blockIdx.x * kClimb, i = b0 + threadIdx.x;
+  sm.seen[threadIdx.x] = 0;
+  __syncthreads();
+  if (i >= P || P < 2) return;
+  float4 lo, hi;
+  tri_box(tri, i, lo, hi);
+  climb(sm, i, b0, lo, hi, tri, bn, bparent, lparent, flags);
+}
+
+// Refit in one launch: the triangle records of both orders from the vertices,
+// and the boxes above them (as k_prep, k_records and k_bottom_up of a build).
+// 100k triangles: 58 us as three launches with every level through global
+// flags, 50 in one with the blocks' own levels in shared memory, 36 with the
+// parent's links loaded ahead and one acquire-release arrival instead of two
+// fences (38 at 512 leaves a block); 1M triangles 196 -> 138 us. What is left is
+// the chain of ~10 levels of L2 round trips.
+__global__ void __launch_bounds__(kClimb) k_refit(const float* __restrict__ verts, const int* __restrict__ cumsum,
+                                                  const uint32_t* __restrict__ order, int P, float4* __restrict__ tri_prim,
+                                                  float4* tri_sorted, BinNode* bn, const int* __restrict__ bparent,
+                                                  const int* __restrict__ lparent, int* flags) {
+  __shared__ ClimbMem sm;
+  const int b0 = blockIdx.x * kClimb, i = b0 + threadIdx.x;
+  sm.seen[threadIdx.x] = 0;
+  __syncthreads();
+  if (i >= P) return;
+  const uint32_t p = order[i];
+  const float* v = verts + 3 * (size_t)cumsum[p];
+  float x[9];
+#pragma unroll
+  for (int k = 0; k < 9; ++k) x[k] = v[k];
+  const float4 a = make_float4(x[0], x[1], x[2], __int_as_float((int)p)), b = make_float4(x[3], x[4], x[5], 0.f),
+               c = make_float4(x[6], x[7], x[8], 0.f);
+  tri_prim[3 * (size_t)p + 0] = a;
+  tri_prim[3 * (size_t)p + 1] = b;
+  tri_prim[3 * (size_t)p + 2] = c;
+  __stcg(tri_sorted + 3 * (size_t)i + 0, a);
+  __stcg(tri_sorted + 3 * (size_t)i + 1, b);
+  __stcg(tri_sorted + 3 * (size_t)i + 2, c);
+  if (P < 2) return;
+  climb(sm, i, b0,
+        make_float4(fminf(a.x, fminf(b.x, c.x)), fminf(a.y, fminf(b.y, c.y)), fminf(a.z, fminf(b.z, c.z)), 0.f),
+        make_float4(fmaxf(a.x, fmaxf(b.x, c.x)), fmaxf(a.y, fmaxf(b.y, c.y)), fmaxf(a.z, fmaxf(b.z, c.z)), 0.f),
+        tri_sorted, bn, bparent, lparent, flags);
 }
 
 // ------------------------------------------------------------- collapse
@@ -605,7 +725,6 @@ cudaError_t launch_collapse(int P, const BinNode* bn, int* levels, int* wbin, in
 cudaError_t Bvh::reserve(int P) {
   if (P <= cap_) return cudaSuccess;
   const size_t n = (size_t)P;
-  const size_t tiles = (n + kSortTile - 1) / kSortTile;
   const size_t wcap = n > 1 ? n - 1 : 1;
   cudaError_t e;
 #define TT_RES(buf, bytes)            \
@@ -618,7 +737,7 @@ cudaError_t Bvh::reserve(int P) {
   TT_RES(vals_, n * 4);
   TT_RES(keys2_, n * 4);
   TT_RES(vals2_, n * 4);
-  TT_RES(hist_, hist_words_for_tiles(tiles) * 4);
+  TT_RES(hist_, sort_pairs_hist_words(P) * 4);
   TT_RES(bnode_, (n > 1 ? n - 1 : 1) * sizeof(BinNode));
   TT_RES(bparent_, (n > 1 ? n - 1 : 1) * 4);
   TT_RES(lparent_, n * 4);
@@ -633,34 +752,6 @@ cudaError_t Bvh::reserve(int P) {
   return cudaSuccess;
 }
 
-cudaError_t Bvh::prep(const float* verts, const int* cumsum, int P, bool with_centroids, cudaStream_t s) {
-  if (with_centroids) {
-    k_bounds_init<<<1, 32, 0, s>>>(bounds_.as<int>());
-    ++launches_;
-  }
-  ++launches_;
-  k_prep<<<blocks_for(P), kBlock, 0, s>>>(verts, cumsum, P, tri_prim_.as<float4>(),
-                                          with_centroids ? centroid_.as<float4>() : nullptr, bounds_.as<int>());
-  return cudaGetLastError();
-}
-
-cudaError_t Bvh::boxes(cudaStream_t s) {
-  const int P = P_;
-  cudaError_t e;
-  if (P >= 2) {
-    if ((e = cudaMemsetAsync(flags_.p, 0, (size_t)(P - 1) * 4, s)) != cudaSuccess) return e;
-    k_bottom_up<<<blocks_for(P), kBlock, 0, s>>>(tri_sorted_.as<float4>(), P, bnode_.as<BinNode>(),
-                                                 bparent_.as<int>(), lparent_.as<int>(), flags_.as<int>());
-    ++launches_;
-  }
-  ++launches_;
-  const int wcap = P > 1 ? P - 1 : 1;
-  const int grid = blocks_for(wcap) < 148 * 8 ? blocks_for(wcap) : 148 * 8;
-  k_wide_boxes<<<grid, kBlock, 0, s>>>(wsrc_.as<int>(), bnode_.as<BinNode>(), tri_sorted_.as<float4>(),
-                                       counters_.as<int>(), wcap, wnodes_.as<float4>());
-  return cudaGetLastError();
-}
-
 cudaError_t Bvh::build(const float* verts, const int* cumsum, int P, cudaStream_t s) {
   built_ = false;
   P_ = P;
@@ -670,20 +761,19 @@ cudaError_t Bvh::build(const float* verts, const int* cumsum, int P, cudaStream_
   }
   cudaError_t e = reserve(P);
   if (e != cudaSuccess) return e;
-  if ((e = prep(verts, cumsum, P, true, s)) != cudaSuccess) return e;
-  // morton + 4 x (hist, scan, scatter) + records + karras + bottom-up + collapse init/levels/total + boxes
-  const int tiles = (P + kSortTile - 1) / kSortTile;
-  launches_ += 1 + 4 * (2 + scan_launches(tiles)) + 1 + (P >= 2 ? 2 : 0) + 1 + (2 + collapse_big_launches(P)) + 1 + 1;
+  // bounds init + prep + morton + 4 x (hist, scan, scatter) + records + karras + bottom-up + collapse init/levels/total + boxes
+  const int tiles = (int)sort_tiles((size_t)P);
+  launches_ += 3 + 4 * (2 + scan_launches(tiles)) + 1 + (P >= 2 ? 2 : 0) + 1 + (2 + collapse_big_launches(P)) + 1 + 1;
+  k_bounds_init<<<1, 32, 0, s>>>(bounds_.as<int>());
+  k_prep<<<blocks_for(P), kBlock, 0, s>>>(verts, cumsum, P, tri_prim_.as<float4>(), centroid_.as<float4>(),
+                                          bounds_.as<int>());
   k_morton<<<blocks_for(P), kBlock, 0, s>>>(centroid_.as<float4>(), bounds_.as<int>(), P, keys_.as<uint32_t>(),
                                             vals_.as<uint32_t>());
   // 30-bit keys: four 8-bit passes, ending back in keys_/vals_
   uint32_t *ka = keys_.as<uint32_t>(), *va = vals_.as<uint32_t>();
   uint32_t *kb = keys2_.as<uint32_t>(), *vb = vals2_.as<uint32_t>();
   for (int pass = 0; pass < 4; ++pass) {
-    const int shift = 8 * pass;
-    k_sort_hist<<<tiles, kBlock, 0, s>>>(ka, P, shift, hist_.as<uint32_t>(), tiles);
-    scan_hist(hist_.as<uint32_t>(), tiles, s);
-    k_sort_scatter<<<tiles, kBlock, 0, s>>>(ka, va, kb, vb, P, shift, hist_.as<uint32_t>(), tiles);
+    sort_pass(ka, va, kb, vb, hist_.as<uint32_t>(), P, 8 * pass, s);
     uint32_t* t;
     t = ka; ka = kb; kb = t;
     t = va; va = vb; vb = t;
@@ -698,7 +788,7 @@ cudaError_t Bvh::build(const float* verts, const int* cumsum, int P, cudaStream_
   // binary boxes are needed by the collapse's area heuristic
   if (P >= 2) {
     if ((e = cudaMemsetAsync(flags_.p, 0, (size_t)(P - 1) * 4, s)) != cudaSuccess) return e;
-    k_bottom_up<<<blocks_for(P), kBlock, 0, s>>>(tri_sorted_.as<float4>(), P, bnode_.as<BinNode>(),
+    k_bottom_up<<<(P + kClimb - 1) / kClimb, kClimb, 0, s>>>(tri_sorted_.as<float4>(), P, bnode_.as<BinNode>(),
                                                  bparent_.as<int>(), lparent_.as<int>(), flags_.as<int>());
   }
   if ((e = launch_collapse(P, bnode_.as<BinNode>(), levels_.as<int>(), wbin_.as<int>(), wsrc_.as<int>(),
@@ -717,12 +807,15 @@ cudaError_t Bvh::build(const float* verts, const int* cumsum, int P, cudaStream_
 cudaError_t Bvh::refit(const float* verts, const int* cumsum, int P, cudaStream_t s) {
   if (!built_ || P != P_) return build(verts, cumsum, P, s);
   if (P <= 0) return cudaSuccess;
-  cudaError_t e;
-  if ((e = prep(verts, cumsum, P, false, s)) != cudaSuccess) return e;
-  ++launches_;
-  k_records<<<blocks_for(P), kBlock, 0, s>>>(vals_.as<uint32_t>(), tri_prim_.as<float4>(), P,
-                                             tri_sorted_.as<float4>());
-  return boxes(s);
+  launches_ += 2;
+  k_refit<<<(P + kClimb - 1) / kClimb, kClimb, 0, s>>>(verts, cumsum, vals_.as<uint32_t>(), P, tri_prim_.as<float4>(),
+                                           tri_sorted_.as<float4>(), bnode_.as<BinNode>(), bparent_.as<int>(),
+                                           lparent_.as<int>(), flags_.as<int>());
+  const int wcap = P > 1 ? P - 1 : 1;
+  const int grid = blocks_for(wcap) < 148 * 8 ? blocks_for(wcap) : 148 * 8;
+  k_wide_boxes<<<grid, kBlock, 0, s>>>(wsrc_.as<int>(), bnode_.as<BinNode>(), tri_sorted_.as<float4>(),
+                                       counters_.as<int>(), wcap, wnodes_.as<float4>());
+  return cudaGetLastError();
 }
 
 // BVH blob: the topology only. Every box (binary nodes' lo/hi, the wide
@@ -895,6 +988,7 @@ int Bvh::load(const void* src, size_t bytes, const float* verts, const int* cums
   h2d(lparent_, p * 4);
   h2d(wsrc_, (size_t)hd.nw * kWide * 4);
   h2d_rows(wnodes_, kWideRefOff, kWideRefBytes, kNodeF4 * sizeof(float4), (size_t)hd.nw);
+  if (e == cudaSuccess) e = cudaMemsetAsync(flags_.p, 0, b * 4, s);  // as a build leaves them
   const int cnt[4] = {hd.nw, 0, 0, 0};
   if (e == cudaSuccess) e = cudaMemcpyAsync(counters_.p, cnt, sizeof(cnt), cudaMemcpyHostToDevice, s);
   // the host blob and cnt may go away on return
@@ -945,7 +1039,7 @@ struct Carver {
 
 BvhStorage carve(char* base, int P, size_t* total) {
   const size_t n = (size_t)(P > 0 ? P : 1);
-  const size_t tiles = (n + kSortTile - 1) / kSortTile;
+  const size_t tiles = sort_tiles(n);
   const size_t inner = n > 1 ? n - 1 : 1;
   Carver c{base};
   BvhStorage st;
@@ -987,12 +1081,9 @@ cudaError_t bvh_build_into(const BvhStorage& st, const float* verts, const int* 
   k_bounds_init<<<1, 32, 0, s>>>(st.bounds);
   k_prep<<<blocks_for(P), kBlock, 0, s>>>(verts, cumsum, P, st.tri_prim, st.centroid, st.bounds);
   k_morton<<<blocks_for(P), kBlock, 0, s>>>(st.centroid, st.bounds, P, st.keys, st.vals);
-  const int tiles = (P + kSortTile - 1) / kSortTile;
   uint32_t *ka = st.keys, *va = st.vals, *kb = st.keys2, *vb = st.vals2;
   for (int pass = 0; pass < 4; ++pass) {
-    k_sort_hist<<<tiles, kBlock, 0, s>>>(ka, P, 8 * pass, st.hist, tiles);
-    scan_hist(st.hist, tiles, s);
-    k_sort_scatter<<<tiles, kBlock, 0, s>>>(ka, va, kb, vb, P, 8 * pass, st.hist, tiles);
+    sort_pass(ka, va, kb, vb, st.hist, P, 8 * pass, s);
     uint32_t* t;
     t = ka; ka = kb; kb = t;
     t = va; va = vb; vb = t;
@@ -1002,7 +1093,7 @@ cudaError_t bvh_build_into(const BvhStorage& st, const float* verts, const int* 
   if (P >= 2) {
     k_karras<<<blocks_for(P - 1), kBlock, 0, s>>>(st.keys, P, bn, st.bparent, st.lparent);
     if ((e = cudaMemsetAsync(st.flags, 0, (size_t)(P - 1) * 4, s)) != cudaSuccess) return e;
-    k_bottom_up<<<blocks_for(P), kBlock, 0, s>>>(st.tri_sorted, P, bn, st.bparent, st.lparent, st.flags);
+    k_bottom_up<<<(P + kClimb - 1) / kClimb, kClimb, 0, s>>>(st.tri_sorted, P, bn, st.bparent, st.lparent, st.flags);
   }
   if ((e = launch_collapse(P, bn, st.levels, st.wbin, st.wsrc, st.wnodes, st.counters, s)) != cudaSuccess) return e;
   const int wcap = P > 1 ? P - 1 : 1;
@@ -1012,23 +1103,21 @@ cudaError_t bvh_build_into(const BvhStorage& st, const float* verts, const int* 
   return cudaGetLastError();
 }
 
-size_t sort_pairs_hist_words(int n) { return hist_words_for_tiles((size_t)((n + kSortTile - 1) / kSortTile)); }
+// (a smaller sort may have more tiles, up to kSortTiles)
+size_t sort_pairs_hist_words(int n) { return hist_words_for_tiles(std::max(sort_tiles((size_t)n), (size_t)kSortTiles)); }
 
 int sort_pairs_launches(int n, int bits) {
   if (n <= 0) return 0;
-  return ((bits + 7) / 8) * (2 + scan_launches((n + kSortTile - 1) / kSortTile));
+  return ((bits + 7) / 8) * (2 + scan_launches((int)sort_tiles((size_t)n)));
 }
 
 cudaError_t sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* keys2, uint32_t* vals2, uint32_t* hist, int n,
                        int bits, bool* in_second, cudaStream_t s) {
   *in_second = false;
   if (n <= 0) return cudaSuccess;
-  const int tiles = (n + kSortTile - 1) / kSortTile;
   uint32_t *ka = keys, *va = vals, *kb = keys2, *vb = vals2;
   for (int shift = 0; shift < bits; shift += 8) {
-    k_sort_hist<<<tiles, kBlock, 0, s>>>(ka, n, shift, hist, tiles);
-    scan_hist(hist, tiles, s);
-    k_sort_scatter<<<tiles, kBlock, 0, s>>>(ka, va, kb, vb, n, shift, hist, tiles);
+    sort_pass(ka, va, kb, vb, hist, n, shift, s);
     uint32_t* t;
     t = ka; ka = kb; kb = t;
     t = va; va = vb; vb = t;

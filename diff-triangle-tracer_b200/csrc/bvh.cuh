@@ -49,8 +49,6 @@ class Bvh {
 
  private:
   cudaError_t reserve(int P);
-  cudaError_t prep(const float* verts, const int* cumsum, int P, bool sorted_only, cudaStream_t s);
-  cudaError_t boxes(cudaStream_t s);
 
   unsigned long long launches_ = 0;
   int P_ = 0;
