@@ -29,8 +29,8 @@ struct tt_tracer {
   int cfg_id = tt::kCfgPackets16;
   std::string err;
   tt::Bvh bvh;
-  tt::DevBuf scratch;  // int[0] tile counter, int[1] status word, u64 stats[kNumStats] from byte 16,
-                       // int[3] secondary-ray queue counters from byte kSecCountOffset
+  tt::DevBuf scratch;  // int[1] status word, u64 stats[kNumStats] from byte 16, int[3] secondary-ray queue
+                       // counters from byte kSecCountOffset, work counters from byte kWorkOffset
   tt::DevBuf sec_rec;  // secondary-ray queue: R * (2^(depth+1) - 1) records
   tt::DevBuf sec_cache;        // hit cache of that ray tree (tt_forward_secondary writes, the adjoint replays)
   size_t sec_cache_bytes = 0;  // its size for the last tree
@@ -49,6 +49,11 @@ namespace {
 
 constexpr int kSecCountOffset = 96;
 static_assert(16 + tt::kNumStats * 8 <= kSecCountOffset, "stats overlap the secondary-ray counters");
+// tile / item counters, one for each launch of an entry point that takes work
+// from one, zeroed together
+constexpr int kWorkOffset = 128, kWorkCounters = 8;
+constexpr size_t kScratchBytes = kWorkOffset + kWorkCounters * sizeof(int);
+static_assert(2 * (tt::kMaxSecDepth + 1) <= kWorkCounters, "a counter for each pass over each level");
 
 int fail(tt_tracer* h, int code, const std::string& msg) {
   if (h) h->err = msg;
@@ -163,7 +168,8 @@ int tt_create(const tt_config* cfg, tt_tracer** out) {
   cudaError_t e;
   if ((e = cudaGetDevice(&h->device)) != cudaSuccess ||
       (e = cudaDeviceGetAttribute(&h->num_sms, cudaDevAttrMultiProcessorCount, h->device)) != cudaSuccess ||
-      (e = h->scratch.reserve(128)) != cudaSuccess || (e = cudaMemset(h->scratch.p, 0, 128)) != cudaSuccess ||
+      (e = h->scratch.reserve(kScratchBytes)) != cudaSuccess ||
+      (e = cudaMemset(h->scratch.p, 0, kScratchBytes)) != cudaSuccess ||
       (e = cudaEventCreate(&h->ev0)) != cudaSuccess || (e = cudaEventCreate(&h->ev1)) != cudaSuccess ||
       (e = cudaEventCreate(&h->ev_mid)) != cudaSuccess) {
     delete h;
@@ -294,7 +300,7 @@ static tt::TraceParams base_params(tt_tracer* h) {
   p.variant = h->cfg.variant;
   p.cfg = h->cfg_id;
   p.count_work = h->count_work ? 1 : 0;
-  p.work = h->scratch.as<int>();
+  p.work = reinterpret_cast<int*>(h->scratch.as<char>() + kWorkOffset);
   p.status = h->scratch.as<int>() + 1;
   p.stats = reinterpret_cast<unsigned long long*>(h->scratch.as<char>() + 16);
   return p;
@@ -369,7 +375,6 @@ static int forward_impl(tt_tracer* h, const tt_fwd_args* a, const tt_view* views
     p.cache_gen = h->bvh_gen;
     p.cache_pool_cap = (uint32_t)cap;
     p.cache_colors = cache_colors_of(a->hit_cache, h->k(), p.cache_rays, cap);
-    TT_CUDA(h, cudaMemsetAsync(a->hit_cache, 0, sizeof(tt::HitCacheHeader), s));
   }
   p.bvh = h->bvh.view();
   p.verts = a->vertices;
@@ -390,13 +395,17 @@ static int forward_impl(tt_tracer* h, const tt_fwd_args* a, const tt_view* views
   p.sph_cy = ex[2];
   p.sph_cz = ex[3];
   p.samples = (int)ex[4];
-  if (a->P > 0) TT_CUDA(h, cudaMemsetAsync(a->max_blending, 0, (size_t)a->P * sizeof(float), s));
+  tt::ZeroList zero;
+  zero.add(p.hit_cache, p.hit_cache ? sizeof(tt::HitCacheHeader) : 0);
+  zero.add(a->max_blending, (size_t)a->P * sizeof(float));
+  zero.add(p.work, 2 * sizeof(int));
+  TT_CUDA(h, tt::launch_zero(zero, s));
+  ++h->trace_launches;
   if (a->debug) TT_CUDA(h, cudaEventRecord(h->ev0, s));
   const bool split = p.hit_cache && h->split_forward;
   if (split) {
     // traversal-only pass: every query of the march into the cache; the
     // shading pass below replays them
-    TT_CUDA(h, cudaMemsetAsync(p.work, 0, sizeof(int), s));
     p.collect_queries = h->collect_queries;
     TT_CUDA(h, tt::launch_collect(p, h->collect_grid, s));
     ++h->trace_launches;
@@ -411,7 +420,7 @@ static int forward_impl(tt_tracer* h, const tt_fwd_args* a, const tt_view* views
     if (p.fwd_pair) ++h->trace_launches;
   }
   if (a->debug) TT_CUDA(h, cudaEventRecord(h->ev_mid, s));
-  TT_CUDA(h, cudaMemsetAsync(p.work, 0, sizeof(int), s));
+  ++p.work;
   TT_CUDA(h, tt::launch_forward(p, h->fwd_grid, s));
   ++h->trace_launches;
   if (a->debug) {
@@ -480,13 +489,15 @@ static int backward_impl(tt_tracer* h, const tt_bwd_args* a, const tt_view* view
     rc = add_view(h, p, views[i]);
     if (rc != TT_OK) return rc;
   }
+  tt::ZeroList zero;
   if (a->P > 0) {
-    TT_CUDA(h, cudaMemsetAsync(a->dL_dtriangle, 0, (size_t)a->num_vertices * 3 * sizeof(float), s));
-    TT_CUDA(h, cudaMemsetAsync(a->dL_dsigma, 0, (size_t)a->P * sizeof(float), s));
-    TT_CUDA(h, cudaMemsetAsync(a->dL_dopacity, 0, (size_t)a->P * sizeof(float), s));
-    if (a->dL_dsh && a->M > 0) TT_CUDA(h, cudaMemsetAsync(a->dL_dsh, 0, (size_t)a->P * a->M * 3 * sizeof(float), s));
-    if (cols) TT_CUDA(h, cudaMemsetAsync(a->dL_dcolors, 0, (size_t)a->P * 3 * sizeof(float), s));
+    zero.add(a->dL_dtriangle, (size_t)a->num_vertices * 3 * sizeof(float));
+    zero.add(a->dL_dsigma, (size_t)a->P * sizeof(float));
+    zero.add(a->dL_dopacity, (size_t)a->P * sizeof(float));
+    if (a->M > 0) zero.add(a->dL_dsh, (size_t)a->P * a->M * 3 * sizeof(float));
+    if (cols) zero.add(a->dL_dcolors, (size_t)a->P * 3 * sizeof(float));
   }
+  zero.add(p.work, sizeof(int));
   p.verts = a->vertices;
   p.cumsum = a->cumsum;
   p.num_points = a->num_points;
@@ -513,7 +524,8 @@ static int backward_impl(tt_tracer* h, const tt_bwd_args* a, const tt_view* view
     p.cache_pool_cap = (uint32_t)cap;
     p.cache_colors = cache_colors_of(const_cast<void*>(a->hit_cache), h->k(), p.cache_rays, cap);
   }
-  TT_CUDA(h, cudaMemsetAsync(p.work, 0, sizeof(int), s));
+  TT_CUDA(h, tt::launch_zero(zero, s));
+  ++h->trace_launches;
   if (a->debug) TT_CUDA(h, cudaEventRecord(h->ev0, s));
   // with a cache, the packet configurations run the adjoint as a pair: a
   // replay-only build (no traversal code, for a complete cache) and the
@@ -846,7 +858,6 @@ int tt_forward_secondary(tt_tracer* h, const tt_fwd_args* a, const tt_secondary*
   p.cache_mode = tt::kCacheWrite;
   p.cache_gen = h->bvh_gen;
   p.cache_pool_cap = (uint32_t)cache_pool_cap(tt::kChunk, R, cache_bytes);
-  TT_CUDA(h, cudaMemsetAsync(h->sec_cache.p, 0, sizeof(tt::HitCacheHeader), s));
   p.bvh = h->bvh.view();
   p.verts = a->vertices;
   p.cumsum = a->cumsum;
@@ -863,8 +874,13 @@ int tt_forward_secondary(tt_tracer* h, const tt_fwd_args* a, const tt_secondary*
   int* count = reinterpret_cast<int*>(h->scratch.as<char>() + kSecCountOffset);
   sec_layout(p.sec, sec, h->sec_rec.as<tt::SecRecord>(), (int)R, count);
   h->sec_depth = -1;  // no valid tree until this call's launches are enqueued
-  if (a->P > 0) TT_CUDA(h, cudaMemsetAsync(a->max_blending, 0, (size_t)a->P * sizeof(float), s));
-  TT_CUDA(h, cudaMemsetAsync(count, 0, (tt::kMaxSecDepth + 1) * sizeof(int), s));
+  tt::ZeroList zero;
+  zero.add(h->sec_cache.p, sizeof(tt::HitCacheHeader));
+  zero.add(a->max_blending, (size_t)a->P * sizeof(float));
+  zero.add(count, (tt::kMaxSecDepth + 1) * sizeof(int));
+  zero.add(p.work, kWorkCounters * sizeof(int));
+  TT_CUDA(h, tt::launch_zero(zero, s));
+  ++h->trace_launches;
   uint32_t *keys = nullptr, *vals = nullptr, *keys2 = nullptr, *vals2 = nullptr, *hist = nullptr;
   if (h->sort_secondary && sec->max_depth > 0) {
     const long long cap = R << sec->max_depth;  // the deepest level's capacity
@@ -897,7 +913,6 @@ int tt_forward_secondary(tt_tracer* h, const tt_fwd_args* a, const tt_secondary*
       // traversal-only pass over the level (the primary rays as warp
       // packets of 16-hit queries, like k_sec_primary; spawned rays lane by
       // lane), then the shading pass replays it
-      TT_CUDA(h, cudaMemsetAsync(p.work, 0, sizeof(int), s));
       if (level == 0) {
         tt::TraceParams q = p;
         q.cfg = tt::kCfgPackets16;
@@ -907,12 +922,13 @@ int tt_forward_secondary(tt_tracer* h, const tt_fwd_args* a, const tt_secondary*
         TT_CUDA(h, tt::launch_sec_collect(p, h->sec_collect_grid, s));
       }
       ++h->trace_launches;
+      ++p.work;
       p.cache_mode = tt::kCacheFill;
     }
-    TT_CUDA(h, cudaMemsetAsync(p.work, 0, sizeof(int), s));
     TT_CUDA(h, level == 0 ? tt::launch_sec_primary(p, h->sec_primary_grid, s)
                           : tt::launch_sec_trace(p, h->sec_trace_grid, s));
     ++h->trace_launches;
+    ++p.work;
   }
   for (int level = sec->max_depth; level >= 0; --level) {
     p.sec.level = level;
@@ -981,12 +997,14 @@ int tt_backward_secondary(tt_tracer* h, const tt_bwd_args* a, const tt_secondary
   v.dL_dothers = a->dL_dothers;
   rc = add_view(h, p, v);
   if (rc != TT_OK) return rc;
+  tt::ZeroList zero;
   if (a->P > 0) {
-    TT_CUDA(h, cudaMemsetAsync(a->dL_dtriangle, 0, (size_t)a->num_vertices * 3 * sizeof(float), s));
-    TT_CUDA(h, cudaMemsetAsync(a->dL_dsigma, 0, (size_t)a->P * sizeof(float), s));
-    TT_CUDA(h, cudaMemsetAsync(a->dL_dopacity, 0, (size_t)a->P * sizeof(float), s));
-    TT_CUDA(h, cudaMemsetAsync(a->dL_dsh, 0, (size_t)a->P * a->M * 3 * sizeof(float), s));
+    zero.add(a->dL_dtriangle, (size_t)a->num_vertices * 3 * sizeof(float));
+    zero.add(a->dL_dsigma, (size_t)a->P * sizeof(float));
+    zero.add(a->dL_dopacity, (size_t)a->P * sizeof(float));
+    zero.add(a->dL_dsh, (size_t)a->P * a->M * 3 * sizeof(float));
   }
+  zero.add(p.work, sizeof(int));
   p.verts = a->vertices;
   p.cumsum = a->cumsum;
   p.num_points = a->num_points;
@@ -1007,11 +1025,11 @@ int tt_backward_secondary(tt_tracer* h, const tt_bwd_args* a, const tt_secondary
       p.sec.bwd_order[l] = h->sec_order.as<uint32_t>() + (size_t)(p.sec.base[l] - h->sec_R);
   if (sec->dL_denv) {
     p.sec.d_env = sec->dL_denv;
-    TT_CUDA(h, cudaMemsetAsync(sec->dL_denv, 0, (size_t)sec->env_h * sec->env_w * 3 * sizeof(float), s));
+    zero.add(sec->dL_denv, (size_t)sec->env_h * sec->env_w * 3 * sizeof(float));
   }
   if (sec->dL_dior && a->P > 0) {
     p.sec.d_ior = sec->dL_dior;
-    TT_CUDA(h, cudaMemsetAsync(sec->dL_dior, 0, (size_t)a->P * sizeof(float), s));
+    zero.add(sec->dL_dior, (size_t)a->P * sizeof(float));
   }
   if (h->sec_cache_bytes > 0) {  // replayed where its header matches (same BVH generation)
     p.hit_cache = h->sec_cache.p;
@@ -1019,7 +1037,8 @@ int tt_backward_secondary(tt_tracer* h, const tt_bwd_args* a, const tt_secondary
     p.cache_gen = h->bvh_gen;
     p.cache_pool_cap = (uint32_t)cache_pool_cap(tt::kChunk, p.cache_rays, h->sec_cache_bytes);
   }
-  TT_CUDA(h, cudaMemsetAsync(p.work, 0, sizeof(int), s));
+  TT_CUDA(h, tt::launch_zero(zero, s));
+  ++h->trace_launches;
   if (a->debug) TT_CUDA(h, cudaEventRecord(h->ev0, s));
   TT_CUDA(h, tt::launch_sec_backward(p, h->sec_bwd_grid, s));
   ++h->trace_launches;

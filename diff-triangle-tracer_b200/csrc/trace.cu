@@ -3643,6 +3643,21 @@ __global__ void __launch_bounds__(kTraceThreads, 4) k_sec_backward(const __grid_
   if ((threadIdx.x & 31) == 0 && s != 0u) atomicAdd(p.stats + kStatReplays, (unsigned long long)s);
 }
 
+// ---------------------------------------------------------------- zero
+__global__ void __launch_bounds__(256) k_zero(const __grid_constant__ ZeroList z) {
+  const size_t i0 = blockIdx.x * (size_t)blockDim.x + threadIdx.x, step = (size_t)gridDim.x * blockDim.x;
+  for (int r = 0; r < z.n; ++r) {
+    uint32_t* p = z.p[r];
+    const size_t words = z.words[r];
+    // 16-byte stores between the ragged ends
+    const size_t head = min(words, (size_t)((4u - (((uintptr_t)p >> 2) & 3u)) & 3u)), quads = (words - head) / 4;
+    uint4* q = reinterpret_cast<uint4*>(p + head);
+    for (size_t i = i0; i < quads; i += step) q[i] = make_uint4(0u, 0u, 0u, 0u);
+    const size_t ragged = words - 4 * quads;
+    if (i0 < ragged) p[i0 < head ? i0 : i0 + 4 * quads] = 0u;
+  }
+}
+
 // ---------------------------------------------------------------- hit stream
 __global__ void __launch_bounds__(kTraceThreads) k_hit_stream(HitStreamParams p) {
   const Smem sm = thread_smem<kStackDepth>();
@@ -3682,6 +3697,15 @@ __global__ void __launch_bounds__(kTraceThreads) k_hit_stream(HitStreamParams p)
 }
 
 }  // namespace
+
+cudaError_t launch_zero(const ZeroList& z, cudaStream_t s) {
+  size_t most = 0;
+  for (int i = 0; i < z.n; ++i) most = std::max(most, (size_t)z.words[i]);
+  if (most == 0) return cudaSuccess;
+  const int grid = (int)std::min<size_t>((most / 4 + 255) / 256 + 1, 148 * 8);
+  k_zero<<<grid, 256, 0, s>>>(z);
+  return cudaGetLastError();
+}
 
 size_t trace_smem_bytes(int cfg) {
   switch (cfg) {

@@ -200,6 +200,22 @@ constexpr int kCfgPackets32 = 2;  // warp packets, 32 hits per query
 constexpr int kCfgLanes24 = 3;    // one ray per lane, 24-entry stack
 constexpr int kNumCfgs = 4;
 
+// Memory an entry point wants zero before its kernels: up to kMaxZero ranges of
+// whole 4-byte words, cleared by one launch (a memset node apiece cost the
+// 100k-triangle training step nine launches of its ~20).
+constexpr int kMaxZero = 8;
+struct ZeroList {
+  uint32_t* p[kMaxZero];
+  unsigned long long words[kMaxZero];
+  int n = 0;
+  void add(void* ptr, size_t bytes) {
+    if (ptr == nullptr || bytes == 0) return;
+    p[n] = static_cast<uint32_t*>(ptr);
+    words[n++] = bytes / 4;
+  }
+};
+cudaError_t launch_zero(const ZeroList& z, cudaStream_t s);
+
 size_t trace_smem_bytes(int cfg);
 // Resident blocks per SM of the forward / adjoint / variant kernels.
 int trace_blocks_per_sm(int which /*0 forward, 1 adjoint, 2 variant, 3 collecting pass*/, int cfg);

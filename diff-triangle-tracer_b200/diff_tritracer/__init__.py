@@ -75,6 +75,7 @@ class _Tracer(torch.autograd.Function):
         ctx.save_for_backward(ray_o, ray_d, triangles_points, sigma, num_points_per_triangle,
                               cumsum_of_points_per_triangle, color, others, colors_precomp, opacities, shs, scaling)
         ctx.mark_non_differentiable(gpu_time, scaling, density_factor, max_blending)
+        ctx.set_materialize_grads(False)  # no zero tensors for outputs without a gradient
         return color, gpu_time, scaling, density_factor, others, max_blending
 
     @staticmethod

@@ -25,6 +25,7 @@ class _Secondary(torch.autograd.Function):
         ctx.save_for_backward(ray_o, ray_d, triangles_points, sigma, num_points, cumsum, opacities, shs, material,
                               ior, env, color, others)
         ctx.mark_non_differentiable(others, max_blending, scaling, density)
+        ctx.set_materialize_grads(False)  # no zero tensors for outputs without a gradient
         return color, others, max_blending, scaling, density
 
     @staticmethod
