@@ -351,12 +351,7 @@ __device__ __forceinline__ void warp_scene(const BvhView& bvh, const WarpStack& 
 // images (ms; as packets / ray by ray): 1M triangles 128^2 3.5 / 5.8, 256^2
 // 1.7 / 5.7; 3M triangles 64^2 22.0 / 9.2, 128^2 8.5 / 9.3, 256^2 3.9 / 9.8;
 // 616k triangles 31 x 38 21.2 / 3.5; 100k triangles 64^2 0.6 / 1.0.
-#ifndef TT_PACKET_MIN
-#define TT_PACKET_MIN 1024.0f
-#endif
-#ifndef TT_PACKET_RATIO
-#define TT_PACKET_RATIO 2.5f
-#endif
+constexpr float kPacketMin = 1024.0f, kPacketRatio = 2.5f;
 
 // Sorts the first n keys of a lane's column, of which the first `done` are in
 // order (insertion: traversal finds hits nearly in order).
@@ -463,8 +458,6 @@ __device__ __forceinline__ unsigned rays_meeting(const float4* slope, float Au, 
   }
   return __brev(~out);
 }
-
-constexpr float kPacketMin = TT_PACKET_MIN, kPacketRatio = TT_PACKET_RATIO;
 
 template <int K>
 __device__ __forceinline__ void packet_query(const BvhView& bvh, const RayW& r, bool want,
@@ -1674,9 +1667,9 @@ __device__ __forceinline__ PairMem pair_mem(unsigned char* base) {
   return pm;
 }
 
-// Packet driver: a warp takes an 8x4-pixel tile, then runs rounds of one
-// packet query (all lanes whose ray is unfinished) and one shading pass until
-// every ray of the tile is done.
+// Packet driver: a warp takes an 8x4-pixel tile (or, of a small image, a part
+// of one: p.parts_log), then runs rounds of one packet query (all lanes whose
+// ray is unfinished) and one shading pass until every ray of it is done.
 __device__ __forceinline__ WarpStack warp_stack(unsigned char* base) {
   base += (size_t)(threadIdx.x >> 5) * kWarpBytes;
   WarpStack ws;
@@ -1711,11 +1704,13 @@ __device__ __forceinline__ void drive_packets(const TraceParams& p, const Smem& 
     int tile = 0;
     if (lane == 0) tile = atomicAdd(p.work, 1);
     tile = __shfl_sync(full, tile, 0);
+    const int part = tile & ((1 << p.parts_log) - 1);
+    tile >>= p.parts_log;
     if (tile >= p.ntiles) break;
     const ViewDesc& v = p.views[find_view(p, tile)];
     const int lt = tile - v.tile_begin;
     const int px = (lt % v.ntx) * 8 + (lane & 7), py = (lt / v.ntx) * 4 + (lane >> 3);
-    bool active = px < v.W && py < v.H;
+    bool active = px < v.W && py < v.H && (lane << p.parts_log) >> 5 == part;
     float3 o = make_float3(0.f, 0.f, 1.f), d = make_float3(0.f, 0.f, 1.f);
     Cursor cur = first_cursor(p.tmin_inclusive);
     long long g = 0;  // hit cache index of the lane's ray
@@ -1822,6 +1817,7 @@ __device__ __forceinline__ Smem packet_smem(unsigned char*& rest) {
 // Traversal configurations the kernels are instantiated for (the autotuner
 // picks one per workload): warp packets with 16 or 32 hits per query, or
 // independent lanes with a 32- or 24-entry stack per ray.
+constexpr int kMaxPartsLog = 5;  // parts of one ray
 template <int CFG>
 struct TraversalCfg;
 template <>
@@ -2672,11 +2668,13 @@ __global__ void __launch_bounds__(kTraceThreads, kAdjointBlocks) k_adjoint(const
     int tile = 0;
     if (lane == 0) tile = atomicAdd(p.work, 1);
     tile = __shfl_sync(full, tile, 0);
+    const int part = tile & ((1 << p.parts_log) - 1);
+    tile >>= p.parts_log;
     if (tile >= p.ntiles) break;
     const ViewDesc& v = p.views[find_view(p, tile)];
     const int lt = tile - v.tile_begin;
     const int px = (lt % v.ntx) * 8 + (lane & 7), py = (lt / v.ntx) * 4 + (lane >> 3);
-    bool active = px < v.W && py < v.H;
+    bool active = px < v.W && py < v.H && (lane << p.parts_log) >> 5 == part;
     Cursor cur = first_cursor(p.tmin_inclusive);
     long long ray_g = 0;
     if (active) {
@@ -3795,8 +3793,21 @@ static_assert(smem_bytes_for<kCfgPackets32, true>() + kExactSmemBytes <= 48 * 10
 inline int replay_grid(int grid) { return grid / kMinBlocks * kReplayBlocks; }
 inline int adjoint_grid(int grid) { return grid / kMinBlocks * kAdjointBlocks; }
 
+// Parts a tile is taken in (log2): an image with fewer tiles than the grid has
+// warps leaves warps without work, and a warp with a few of a tile's rays walks
+// less for a narrower frustum. Whole tiles / parts: 3M triangles, 64 x 64
+// 7.8 / 1.2 ms; 616k, 31 x 38 3.4 / 0.28 ms; training step of 1M, 128 x 160
+// 3.9 / 1.9 ms; parts of at least 8 rays 2.4, 1.1 and 1.9 ms.
+inline TraceParams with_parts(const TraceParams& p, int grid) {
+  TraceParams q = p;
+  const long long warps = (long long)grid * (kTraceThreads / 32);
+  while (q.parts_log < kMaxPartsLog && ((long long)q.ntiles << (q.parts_log + 1)) <= warps) ++q.parts_log;
+  return q;
+}
+
 template <int MODE>
-cudaError_t launch_forward_t(const TraceParams& p, int grid, cudaStream_t s) {
+cudaError_t launch_forward_t(const TraceParams& in, int grid, cudaStream_t s) {
+  const TraceParams p = with_parts(in, grid);
   const size_t extra = MODE == kShadeExact ? kExactSmemBytes : 0;
   if (p.fwd_pair) {
     if (p.cfg == kCfgPackets16)
@@ -3814,7 +3825,8 @@ cudaError_t launch_forward_t(const TraceParams& p, int grid, cudaStream_t s) {
 }
 
 template <int MODE>
-cudaError_t launch_backward_t(const TraceParams& p, int grid, cudaStream_t s) {
+cudaError_t launch_backward_t(const TraceParams& in, int grid, cudaStream_t s) {
+  const TraceParams p = with_parts(in, grid);
   if (p.bwd_pair) {
     if (p.cfg == kCfgPackets16)
       k_adjoint<16, MODE><<<adjoint_grid(grid), kTraceThreads, adjoint_smem<16, MODE>(), s>>>(p);
@@ -3830,7 +3842,8 @@ cudaError_t launch_backward_t(const TraceParams& p, int grid, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_collect(const TraceParams& p, int grid, cudaStream_t s) {
+cudaError_t launch_collect(const TraceParams& in, int grid, cudaStream_t s) {
+  const TraceParams p = with_parts(in, grid);
   switch (p.cfg) {
     case kCfgPackets16: k_collect<kCfgPackets16><<<grid, kTraceThreads, smem_bytes_for<kCfgPackets16>(), s>>>(p); break;
     case kCfgPackets32: k_collect<kCfgPackets32><<<grid, kTraceThreads, smem_bytes_for<kCfgPackets32>(), s>>>(p); break;
@@ -3882,7 +3895,8 @@ cudaError_t launch_sec_collect(const TraceParams& p, int grid, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_sec_primary(const TraceParams& p, int grid, cudaStream_t s) {
+cudaError_t launch_sec_primary(const TraceParams& in, int grid, cudaStream_t s) {
+  const TraceParams p = with_parts(in, grid);
   k_sec_primary<<<grid, kTraceThreads, smem_bytes_for<kCfgPackets16>(), s>>>(p);
   return cudaGetLastError();
 }

@@ -160,6 +160,7 @@ struct TraceParams {
   int count_work;       // count node visits and triangle tests (tt_stats), off by default
   int bwd_pair;         // adjoint launched as a replay-only / traversing pair: one of the two works
   int fwd_pair;         // shading pass of the split forward launched as such a pair
+  int parts_log;  // log2 of the parts a tile is taken in (packet drivers)
   int* work;    // tile counter, zero at launch
   int* status;  // kStatus* bits
   unsigned long long* stats;  // forward counters, kNumStats of them (add_stats in trace.cu)
