@@ -2420,9 +2420,7 @@ __device__ __forceinline__ void hit_grads(const TraceParams& p, uint32_t prim, c
     window_bwd(g, dL_dphi, dL_dn, gv);
 }
 
-// Scatters one blended hit's vertex and colour gradients.
-__device__ __forceinline__ void scatter_hit(const TraceParams& p, uint32_t prim, float w, float g0, float g1, float g2,
-                                            float3 raw, const float (&B)[16], const float3 (&gv)[3]) {
+__device__ __forceinline__ void scatter_vertices(const TraceParams& p, uint32_t prim, const float3 (&gv)[3]) {
   float* dt = p.d_tri + 3 * (size_t)__ldg(p.cumsum + prim);
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
@@ -2430,6 +2428,12 @@ __device__ __forceinline__ void scatter_hit(const TraceParams& p, uint32_t prim,
     red_add(dt + 3 * k + 1, gv[k].y);
     red_add(dt + 3 * k + 2, gv[k].z);
   }
+}
+
+// Scatters one blended hit's vertex and colour gradients.
+__device__ __forceinline__ void scatter_hit(const TraceParams& p, uint32_t prim, float w, float g0, float g1, float g2,
+                                            float3 raw, const float (&B)[16], const float3 (&gv)[3]) {
+  scatter_vertices(p, prim, gv);
   if (p.cols) {
     red_add(p.d_cols + 3 * prim + 0, g0 * w);
     red_add(p.d_cols + 3 * prim + 1, g1 * w);
@@ -3467,9 +3471,8 @@ struct SecBwdShader {
   const ViewDesc* v;
   int ridx, pix, level;
   float3 o, d;
-  float Cf0, Cf1, Cf2, Df, Nf0, Nf1, Nf2;
   float g0, g1, g2, gD, gN0, gN1, gN2;
-  float C0, C1, C2, N0, N1, N2, D, T;
+  float F, S, T;  // as RayGrads::F and the running sum beside it
   bool spawned;
 
   __device__ explicit SecBwdShader(const TraceParams& params) : p(params), v(&params.views[0]) {}
@@ -3494,30 +3497,28 @@ struct SecBwdShader {
       ro = make_float3(v->ray_o[3 * pix], v->ray_o[3 * pix + 1], v->ray_o[3 * pix + 2]);
       rd = make_float3(v->ray_d[3 * pix], v->ray_d[3 * pix + 1], v->ray_d[3 * pix + 2]);
       tau = 1.0f;
-      Df = __ldg(v->others + kDepthCh * HW + pix);
-      Nf0 = __ldg(v->others + (kNormalCh + 0) * HW + pix);
-      Nf1 = __ldg(v->others + (kNormalCh + 1) * HW + pix);
-      Nf2 = __ldg(v->others + (kNormalCh + 2) * HW + pix);
-      gD = __ldg(v->dL_doth + kDepthCh * HW + pix);
+      // The exact adjoint differentiates the outputs the passes compute: the
+      // depth channel is 0 there (as in the reference), so it has no gradient
+      gD = p.mode == kShadeExact ? 0.f : __ldg(v->dL_doth + kDepthCh * HW + pix);
       gN0 = __ldg(v->dL_doth + (kNormalCh + 0) * HW + pix);
       gN1 = __ldg(v->dL_doth + (kNormalCh + 1) * HW + pix);
       gN2 = __ldg(v->dL_doth + (kNormalCh + 2) * HW + pix);
+      F = gD * __ldg(v->others + kDepthCh * HW + pix) + gN0 * __ldg(v->others + (kNormalCh + 0) * HW + pix) +
+          gN1 * __ldg(v->others + (kNormalCh + 1) * HW + pix) + gN2 * __ldg(v->others + (kNormalCh + 2) * HW + pix);
     } else {
       ro = make_float3(r->o[0], r->o[1], r->o[2]);
       rd = make_float3(r->d[0], r->d[1], r->d[2]);
       pix = r->pixel;
       tau = r->tau;
-      Df = Nf0 = Nf1 = Nf2 = gD = gN0 = gN1 = gN2 = 0.f;
+      F = gD = gN0 = gN1 = gN2 = 0.f;
     }
-    Cf0 = r->L[0];
-    Cf1 = r->L[1];
-    Cf2 = r->L[2];
     g0 = tau * __ldg(v->dL_dpix + pix);
     g1 = tau * __ldg(v->dL_dpix + HW + pix);
     g2 = tau * __ldg(v->dL_dpix + 2 * HW + pix);
+    F += g0 * r->L[0] + g1 * r->L[1] + g2 * r->L[2];
     o = ro;
     d = rd;
-    C0 = C1 = C2 = N0 = N1 = N2 = D = 0.f;
+    S = 0.f;
     T = 1.0f;
     spawned = false;
   }
@@ -3536,13 +3537,13 @@ struct SecBwdShader {
     const float w = alpha * T;
     const SecParams& s = p.sec;
     float c0, c1, c2;
-    float raw0 = 0.f, raw1 = 0.f, raw2 = 0.f;
+    float3 raw = make_float3(0.f, 0.f, 0.f);
     float B[16];
     const bool spawn = !spawned && level < s.max_depth && __ldg(s.material + prim) == 1;
     if (spawn) {
       spawned = true;
       const SecRecord* r = s.rec + ridx;
-      const float F = r->F;
+      const float Fr = r->F;
       float lr[3] = {0.f, 0.f, 0.f}, lt[3] = {0.f, 0.f, 0.f};
       if (r->child_r >= 0) {
         const SecRecord* c = s.rec + s.base[level + 1] + r->child_r;
@@ -3556,71 +3557,33 @@ struct SecBwdShader {
         lt[1] = c->L[1];
         lt[2] = c->L[2];
       }
-      c0 = F * lr[0] + (1.0f - F) * lt[0];
-      c1 = F * lr[1] + (1.0f - F) * lt[1];
-      c2 = F * lr[2] + (1.0f - F) * lt[2];
+      c0 = Fr * lr[0] + (1.0f - Fr) * lt[0];
+      c1 = Fr * lr[1] + (1.0f - Fr) * lt[1];
+      c2 = Fr * lr[2] + (1.0f - Fr) * lt[2];
       if (s.d_ior && r->child_t >= 0) {  // a refracting hit: the colour depends on ior through F
         const float dL_dF = w * (g0 * (lr[0] - lt[0]) + g1 * (lr[1] - lt[1]) + g2 * (lr[2] - lt[2]));
-        red_add(s.d_ior + prim, dL_dF * fresnel_dF_dior(__ldg(s.ior + prim), F));
+        red_add(s.d_ior + prim, dL_dF * fresnel_dF_dior(__ldg(s.ior + prim), Fr));
       }
     } else {
       sh_basis(unit(d), p.sh_degree, B);
-      const float3 raw = sh_raw(p.shs, p.M, (int)prim, p.sh_degree, B);
-      raw0 = raw.x;
-      raw1 = raw.y;
-      raw2 = raw.z;
+      raw = sh_raw(p.shs, p.M, (int)prim, p.sh_degree, B);
       c0 = fmaxf(raw.x, 0.f);
       c1 = fmaxf(raw.y, 0.f);
       c2 = fmaxf(raw.z, 0.f);
     }
-    C0 += c0 * w;
-    C1 += c1 * w;
-    C2 += c2 * w;
-    N0 += g.n.x * w;
-    N1 += g.n.y * w;
-    N2 += g.n.z * w;
-    D += w * g.t;
-    const float inv1a = 1.0f / (1.0f - alpha);
-    float dL_dalpha = g0 * (T * c0 - (Cf0 - C0) * inv1a) + g1 * (T * c1 - (Cf1 - C1) * inv1a) +
-                      g2 * (T * c2 - (Cf2 - C2) * inv1a);
-    // The exact adjoint differentiates the outputs the passes compute: the
-    // depth channel is 0 there (as in the reference), so it has no gradient,
-    // and a clamped alpha passes none; the reference-style adjoint keeps
-    // backward.cu's depth term and differentiates through the clamp.
-    const bool exact = p.mode == kShadeExact;
-    if (!exact) dL_dalpha += gD * (T * g.t - (Df - D) * inv1a);
-    dL_dalpha += gN0 * (T * g.n.x - (Nf0 - N0) * inv1a) + gN1 * (T * g.n.y - (Nf1 - N1) * inv1a) +
-                 gN2 * (T * g.n.z - (Nf2 - N2) * inv1a);
-    const bool live = !exact || opacity * g.Cx < kAlphaMax;
-    const float dL_dC = live ? opacity * dL_dalpha : 0.0f;
-    if (live) red_add(p.d_opac + prim, dL_dalpha * g.Cx);
-    if (g.phi_final > 0.0f) red_add(p.d_sigma + prim, dL_dC * g.Cx * logf(g.phi_final));
-    const float dL_dphi = sig / g.phi_max * dL_dC * g.Cx;
+    const float q = g0 * c0 + g1 * c1 + g2 * c2 + gD * g.t + gN0 * g.n.x + gN1 * g.n.y + gN2 * g.n.z;
+    S += w * q;
+    const float dL_dalpha = T * q - (F - S) * (1.0f / (1.0f - alpha));
+    const float3 dL_dn = make_float3(gN0 * w, gN1 * w, gN2 * w);
     float3 gv[3];
-    if (exact)  // the full chain rule of the window function and the face normal; spawn geometry held constant
-      window_bwd_exact(g, d, dL_dphi, dL_dC * sig * g.Cx, make_float3(gN0 * w, gN1 * w, gN2 * w), 0.0f, gv);
+    if (p.mode == kShadeExact)  // the full chain rule of the window function and the face normal; spawn geometry held constant
+      hit_grads<kShadeExact>(p, prim, g, d, sig, opacity, dL_dalpha, 0.0f, dL_dn, gv);
     else
-      window_bwd(g, dL_dphi, make_float3(gN0 * w, gN1 * w, gN2 * w), gv);
-    float* dt = p.d_tri + 3 * (size_t)__ldg(p.cumsum + prim);
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      red_add(dt + 3 * k + 0, gv[k].x);
-      red_add(dt + 3 * k + 1, gv[k].y);
-      red_add(dt + 3 * k + 2, gv[k].z);
-    }
-    if (!spawn) {
-      const float e0 = raw0 < 0.f ? 0.f : g0 * w, e1 = raw1 < 0.f ? 0.f : g1 * w, e2 = raw2 < 0.f ? 0.f : g2 * w;
-      float* dsh = p.d_sh + (size_t)prim * p.M * 3;
-      const int n = sh_count(p.sh_degree);
-#pragma unroll
-      for (int k = 0; k < 16; ++k) {
-        if (k < n) {
-          red_add(dsh + 3 * k + 0, B[k] * e0);
-          red_add(dsh + 3 * k + 1, B[k] * e1);
-          red_add(dsh + 3 * k + 2, B[k] * e2);
-        }
-      }
-    }
+      hit_grads<kShadeRef>(p, prim, g, d, sig, opacity, dL_dalpha, 0.0f, dL_dn, gv);
+    if (spawn)
+      scatter_vertices(p, prim, gv);
+    else
+      scatter_hit(p, prim, w, g0, g1, g2, raw, B, gv);
     T = test_T;
     return false;
   }
