@@ -88,6 +88,20 @@ struct Range {
 };
 #define TT_RANGE() const Range tt_range_(__func__)
 
+// Makes a device current for a scope.
+struct OnDevice {
+  int before = 0;
+  bool moved = false;
+  explicit OnDevice(int device) {
+    moved = cudaGetDevice(&before) == cudaSuccess && before != device && cudaSetDevice(device) == cudaSuccess;
+  }
+  ~OnDevice() {
+    if (moved) cudaSetDevice(before);
+  }
+  OnDevice(const OnDevice&) = delete;
+  OnDevice& operator=(const OnDevice&) = delete;
+};
+
 int accel_step(tt_tracer* h, const float* verts, int num_vertices, const int* cumsum, int P, int mode,
                cudaStream_t s) {
   TT_REQUIRE(h, mode == TT_BUILD || mode == TT_REFIT || mode == TT_KEEP, "rebuild_gas must be 0, 1 or 2");
@@ -194,7 +208,8 @@ int tt_set_traversal(tt_tracer* h, int traversal, int k, int stack_depth) {
   TT_REQUIRE(h, traversal >= TT_TRAVERSAL_AUTO && traversal <= TT_TRAVERSAL_LANES, "unknown traversal mode");
   TT_REQUIRE(h, k == 0 || k == 16 || k == 32, "k must be 16 or 32");
   TT_REQUIRE(h, stack_depth == 0 || stack_depth == 24 || stack_depth == 32, "stack_depth must be 24 or 32");
-  // sphere variants bend rays incoherently: they always trace lane by lane
+  // sphere variants bend rays incoherently: their queries take (node,
+  // ray) pairs, whatever the stack depth
   const bool lanes = traversal == TT_TRAVERSAL_LANES || h->cfg.variant != TT_VARIANT_PLAIN;
   TT_REQUIRE(h, !(lanes && k == 32), "k = 32 needs packet traversal");
   TT_REQUIRE(h, lanes || stack_depth == 0 || stack_depth == 32, "stack_depth applies to lane traversal");
@@ -203,6 +218,7 @@ int tt_set_traversal(tt_tracer* h, int traversal, int k, int stack_depth) {
     id = stack_depth == 24 ? tt::kCfgLanes24 : tt::kCfgLanes32;
   else
     id = k == 32 ? tt::kCfgPackets32 : tt::kCfgPackets16;
+  const OnDevice on(h->device);  // kernel attributes and occupancy are the handle's device's
   TT_CUDA(h, tt::trace_init(id, shade_mode(h)));
   h->cfg.traversal = traversal;
   h->cfg.k = k;
@@ -911,8 +927,8 @@ int tt_forward_secondary(tt_tracer* h, const tt_fwd_args* a, const tt_secondary*
     p.cache_mode = tt::kCacheWrite;
     if (h->split_forward) {
       // traversal-only pass over the level (the primary rays as warp
-      // packets of 16-hit queries, like k_sec_primary; spawned rays lane by
-      // lane), then the shading pass replays it
+      // packets of 16-hit queries, like k_sec_primary; spawned rays as
+      // (node, ray) pairs), then the shading pass replays it
       if (level == 0) {
         tt::TraceParams q = p;
         q.cfg = tt::kCfgPackets16;

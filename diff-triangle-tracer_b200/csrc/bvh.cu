@@ -80,8 +80,8 @@ __global__ void k_bounds_init(int* b) {
   else if (threadIdx.x < 6) b[threadIdx.x] = (int)0x80000000;
 }
 
-// Triangle records in primitive order (and, when `cen` is set, centroids and
-// their bounds for the Morton quantisation).
+// Triangle records in primitive order, centroids, and the centroids' bounds for
+// the Morton quantisation.
 __global__ void k_prep(const float* __restrict__ verts, const int* __restrict__ cumsum, int P,
                        float4* __restrict__ tri_prim, float4* __restrict__ cen, int* __restrict__ bounds) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
@@ -101,9 +101,8 @@ __global__ void k_prep(const float* __restrict__ verts, const int* __restrict__ 
       const float hi = fmaxf(x[a], fmaxf(x[3 + a], x[6 + a]));
       c[a] = 0.5f * (lo + hi);
     }
-    if (cen) cen[p] = make_float4(c[0], c[1], c[2], 0.f);
+    cen[p] = make_float4(c[0], c[1], c[2], 0.f);
   }
-  if (!cen) return;
   // block reduction of the centroid bounds, then one atomic per block
   __shared__ int s_lo[3][kBlock / 32], s_hi[3][kBlock / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
