@@ -2581,33 +2581,19 @@ __global__ void __launch_bounds__(kTraceThreads, kMinBlocks) k_backward(const __
   if ((threadIdx.x & 31) == 0 && s != 0u) atomicAdd(p.stats + kStatReplays, (unsigned long long)s);
 }
 
-// Inclusive scans over the lanes of a segment (first lane `seg`).
-__device__ __forceinline__ float seg_product(float v, int lane, int seg) {
-#pragma unroll
-  for (int i = 1; i < 32; i <<= 1) {
-    const float u = __shfl_up_sync(0xFFFFFFFFu, v, i);
-    if (lane - i >= seg) v *= u;
-  }
-  return v;
-}
-__device__ __forceinline__ float seg_sum(float v, int lane, int seg) {
-#pragma unroll
-  for (int i = 1; i < 32; i <<= 1) {
-    const float u = __shfl_up_sync(0xFFFFFFFFu, v, i);
-    if (lane - i >= seg) v += u;
-  }
-  return v;
-}
-
 // The adjoint over a complete hit cache, a lane per hit instead of per ray.
 // Ray by ray, a warp's lanes run as many steps as its longest ray, 17 of 32
 // lanes at work on the benchmark's clouds, each step waiting on its gathers.
 // Here each ray's march only lists its next hits (kVisits a round); the lists
 // of the tile's rays are laid end to end and taken 32 at a time, and what a
 // hit needs of the ones before it on its ray, the transmittance and the sum
-// of w q, are two segmented scans, carried from one step to the next in
-// shared memory. A ray ends at the first hit whose product falls below the
-// cut-off.
+// of w q, run along the ray's lanes and are carried from one step to the next
+// in shared memory. A ray ends at the first hit whose transmittance falls below
+// the cut-off; the transmittance is multiplied hit by hit, in the forward's
+// order, because a product that rounds differently ends a ray that lies on the
+// cut-off elsewhere than the forward did, where the cache holds no next query.
+// A ray has at most kVisits lanes of a step, so that chain is as short as the
+// scan of the sums.
 //
 // What bounds it then is L2's handling of the reductions: 23 a hit (12 of 16
 // bytes, the others of 4), each a request and a sector of its own when every
@@ -2617,11 +2603,23 @@ __device__ __forceinline__ float seg_sum(float v, int lane, int seg) {
 // sectors, ~5 requests and 10 sectors a hit.
 //
 // Measured (ms; ray by ray / a lane per hit / regrouped reductions): 1M
-// triangles, 4 views of 800^2, 28M blended hits 4.2 / 4.3 / 3.2; 3M triangles,
-// 16 views, 180M hits 39.0 / 38.6 / 22.1; exact adjoint of 200k triangles
-// 0.24 / 0.18 / 0.19. It issues on 46 % of cycles with L2 39 % and DRAM 16 %
+// triangles, 4 views of 800^2, 28M blended hits 4.2 / 4.3 / 2.9; 3M triangles,
+// 16 views, 180M hits 39.0 / 38.6 / 20.5; exact adjoint of 200k triangles
+// 0.24 / 0.18 / 0.18. (Scans over the whole warp instead of a ray's lanes: 3.2 and
+// 22.1.) It issues on 46 % of cycles with L2 39 % and DRAM 16 %
 // busy: bound by instructions and their latency at 16 warps per SM.
 constexpr int kVisits = 6;
+
+// Inclusive sum over the lanes of a segment (first lane `seg`) of at most 8.
+__device__ __forceinline__ float seg_sum(float v, int lane, int seg) {
+  static_assert(kVisits <= 8, "a segment is a ray's hits of one round");
+#pragma unroll
+  for (int i = 1; i < 8; i <<= 1) {
+    const float u = __shfl_up_sync(0xFFFFFFFFu, v, i);
+    if (lane - i >= seg) v += u;
+  }
+  return v;
+}
 
 struct AdjointMem {
   float4* ray;          // [4][32]: o, gD | d, F | g, T | gN, S (T < 0: the ray has ended)
@@ -2799,10 +2797,15 @@ __global__ void __launch_bounds__(kTraceThreads, kAdjointBlocks) k_adjoint(const
             if (alpha < kAlphaMin) alpha = 0.f;
           }
           // transmittance in front of and behind the hit
-          const float prod = seg_product(1.0f - alpha, lane, seg);
-          const float prev = __shfl_up_sync(full, prod, 1);
-          const float T = lane == seg ? T0 : T0 * prev;
-          const float test_T = T * (1.0f - alpha);
+          float T = T0, test_T = T0 * (1.0f - alpha);
+#pragma unroll
+          for (int i = 1; i < kVisits; ++i) {
+            const float u = __shfl_up_sync(full, test_T, 1);
+            if (lane - seg == i) {
+              T = u;
+              test_T = T * (1.0f - alpha);
+            }
+          }
           const unsigned ended = __ballot_sync(full, on && test_T < kTMin);
           const bool dead = (ended & (full << seg) & (full >> (31 - lane))) != 0u;
           const bool blend = on && alpha > 0.f && !dead;
