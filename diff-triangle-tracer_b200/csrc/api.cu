@@ -22,7 +22,7 @@ struct tt_tracer {
   bool split_forward = true;  // plain forward with a hit cache: collecting pass + shading pass
   int collect_queries = 2;    // queries a ray's collecting pass stores at most (0 = all)
   bool count_work = false;    // node visits and triangle tests counted into the stats
-  bool sort_secondary = true; // secondary passes: spawned rays traced in sorted order
+  int sort_secondary = -1;    // secondary passes: spawned rays traced in sorted order (1), never (0), by size (-1)
   tt::DevBuf sec_sort;        // their sort keys / indices (2 x 2 x 4R words) and the sort's histogram
   tt::DevBuf sec_order;       // each spawned level's trace order, kept for the adjoint
   bool sec_sorted = false;    // the last secondary forward sorted its spawned levels
@@ -235,7 +235,7 @@ int tt_set_option(tt_tracer* h, int option, int value) {
   if (!h) return TT_ERR_INVALID;
   switch (option) {
     case TT_OPT_SPLIT_FORWARD: h->split_forward = value != 0; return TT_OK;
-    case TT_OPT_SORT_SECONDARY: h->sort_secondary = value != 0; return TT_OK;
+    case TT_OPT_SORT_SECONDARY: h->sort_secondary = value != 0 ? 1 : 0; return TT_OK;
     case TT_OPT_WORK_COUNTERS: h->count_work = value != 0; return TT_OK;
     case TT_OPT_COLLECT_QUERIES:
       TT_REQUIRE(h, value >= 0, "collect_queries must be >= 0");
@@ -898,7 +898,15 @@ int tt_forward_secondary(tt_tracer* h, const tt_fwd_args* a, const tt_secondary*
   TT_CUDA(h, tt::launch_zero(zero, s));
   ++h->trace_launches;
   uint32_t *keys = nullptr, *vals = nullptr, *keys2 = nullptr, *vals2 = nullptr, *hist = nullptr;
-  if (h->sort_secondary && sec->max_depth > 0) {
+  // Pairs of (node, ray) leave a warp little to gain from neighbouring rays; what
+  // the sort still saves is L2 misses, and it costs four passes a level. A step,
+  // sorted against in spawn order (ms): 20k triangles, 203 x 151 pixels 0.45 /
+  // 0.34, 1024 x 1024 1.13 / 0.93; 500k, 256 x 256 4.3 / 3.2, 800 x 800 10.3 / 9.6,
+  // 1.28M pixels 17.9 / 17.6, 2.56M 33.6 / 33.8; 2M, 256 x 256 55.8 / 36.4, 1.28M
+  // 249 / 254, 2.56M 465 / 514.
+  constexpr long long kSortPixels = 1 << 20;
+  const bool sorts = h->sort_secondary < 0 ? R > kSortPixels : h->sort_secondary != 0;
+  if (sorts && sec->max_depth > 0) {
     const long long cap = R << sec->max_depth;  // the deepest level's capacity
     const size_t hw = tt::sort_pairs_hist_words((int)cap);
     TT_CUDA(h, h->sec_sort.reserve((size_t)(4 * cap) * 4 + hw * 4));

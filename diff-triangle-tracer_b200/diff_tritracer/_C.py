@@ -418,8 +418,8 @@ class OptixTracer:
 
     def set_sort_secondary(self, on: bool = True):
         """Trace each level of spawned secondary rays sorted by direction
-        (octahedral bins) and origin (default) or in spawn order (False). The results
-        are the same."""
+        (octahedral bins) and origin, or in spawn order (False). Until this is
+        called, images of more than 2^20 pixels sort. The results are the same."""
         check(self._h, lib.tt_set_option(self._h, _lib.TT_OPT_SORT_SECONDARY, 1 if on else 0))
 
     def _scene_fwd_args(self, triangles_points, sigma, num_points_per_triangle, cumsum_of_points_per_triangle,
