@@ -840,9 +840,11 @@ size_t blob_bytes(int P, int nw) {
 
 // Host check of a blob's contents before anything reaches the device: every
 // index in range, the Morton order a permutation, the binary hierarchy a
-// tree rooted at node 0 whose parent links match its child links (the
-// refit's bottom-up pass walks them), and every wide child reference
-// pointing to a later wide node (so the wide hierarchy has no cycle).
+// tree rooted at node 0 whose parent links match its child links and whose
+// nodes are numbered as a build numbers them (the refit's bottom-up pass walks
+// the links, and finds a block's nodes and their slots in shared memory by a
+// node's number and leaf range), and every wide child reference pointing
+// to a later wide node (so the wide hierarchy has no cycle).
 bool blob_contents_valid(const char* in, int P, int nw) {
   const size_t p = (size_t)P, b = P > 1 ? (size_t)P - 1 : 1;
   const uint32_t* vals = reinterpret_cast<const uint32_t*>(in);
@@ -857,33 +859,30 @@ bool blob_contents_valid(const char* in, int P, int nw) {
     seen[vals[i]] = 1;
   }
   if (P >= 2) {
-    const int nb = P - 1;
-    std::vector<char> leaf_seen(p, 0), node_seen(b, 0);
+    // Every node's leaf range follows from the root's: [first, last] splits
+    // behind leaf gamma into the children's ranges, a child of one leaf is that
+    // leaf, any other is node gamma on the left and gamma + 1 on the right, one end
+    // of its own range. So each node is met at most once, and a tree of P leaves
+    // meets them all.
+    if (bparent[0] != -1 || topo[2] != 0 || topo[3] != P - 1) return false;
     std::vector<int> todo{0};
-    if (bparent[0] != -1) return false;
-    int nodes = 0, leaves = 0;
     while (!todo.empty()) {
       const int n = todo.back();
       todo.pop_back();
-      if (node_seen[n]) return false;
-      node_seen[n] = 1;
-      ++nodes;
-      const int* t = topo + 4 * (size_t)n;
-      if (t[2] < 0 || t[3] >= P || t[2] >= t[3]) return false;
+      const int* t = topo + 4 * (size_t)n;  // its range was checked with its parent (the root's above)
+      const int gamma = t[0] >= 0 ? t[0] : ~t[0];
+      if (gamma < t[2] || gamma >= t[3]) return false;
       for (int c = 0; c < 2; ++c) {
-        const int ch = t[c];
-        if (ch >= 0) {
-          if (ch >= nb || bparent[ch] != n) return false;
-          todo.push_back(ch);
+        const int lo = c ? gamma + 1 : t[2], hi = c ? t[3] : gamma, at = gamma + c;
+        if (lo == hi) {
+          if (t[c] != ~lo || lparent[lo] != n) return false;
         } else {
-          const int l = ~ch;
-          if (l >= P || leaf_seen[l] || lparent[l] != n) return false;
-          leaf_seen[l] = 1;
-          ++leaves;
+          const int* u = topo + 4 * (size_t)at;  // (lo < hi <= P - 1, so at is an inner node)
+          if (t[c] != at || bparent[at] != n || u[2] != lo || u[3] != hi) return false;
+          todo.push_back(at);
         }
       }
     }
-    if (nodes != nb || leaves != P) return false;
   }
   for (size_t i = 0; i < (size_t)nw * kWide; ++i) {
     const int v = wsrc[i];
