@@ -1150,12 +1150,16 @@ __device__ __forceinline__ void sh_basis(float3 u, int deg, float (&B)[16]) {
 
 __device__ __forceinline__ int sh_count(int deg) { return (deg + 1) * (deg + 1); }
 
+// 16 coefficients of 3 channels are rows of 192 bytes, taken 16 bytes at a time
+// where the array starts on such a boundary: a caller's may start at any float.
+__device__ __forceinline__ bool on_16_bytes(const float* a) { return (reinterpret_cast<uintptr_t>(a) & 15u) == 0; }
+
 // RGB = sum_k B_k * sh_k + 0.5 (before the clamp at 0).
 __device__ __forceinline__ float3 sh_raw(const float* __restrict__ shs, int M, int prim, int deg, const float (&B)[16]) {
   const float* base = shs + (size_t)prim * M * 3;
   float r = 0.f, g = 0.f, b = 0.f;
-  if (M == 16 && deg == 3) {
-    const float4* q = reinterpret_cast<const float4*>(base);  // 192-byte rows, 16-byte aligned
+  if (M == 16 && deg == 3 && on_16_bytes(shs)) {
+    const float4* q = reinterpret_cast<const float4*>(base);
 #pragma unroll
     for (int i = 0; i < 12; ++i) {
       const float4 w = __ldg(q + i);
@@ -2468,7 +2472,7 @@ __device__ __forceinline__ void scatter_hit(const TraceParams& p, uint32_t prim,
   const float e0 = raw.x < 0.f ? 0.f : g0 * w, e1 = raw.y < 0.f ? 0.f : g1 * w, e2 = raw.z < 0.f ? 0.f : g2 * w;
   float* dsh = p.d_sh + (size_t)prim * p.M * 3;
   const int n = sh_count(p.sh_degree);
-  if (p.M == 16 && n == 16) {
+  if (p.M == 16 && n == 16 && on_16_bytes(p.d_sh)) {
 #pragma unroll
     for (int q = 0; q < 12; ++q) {
       float v4[4];
@@ -2686,7 +2690,7 @@ __global__ void __launch_bounds__(kTraceThreads, kAdjointBlocks) k_adjoint(const
     am.list = reinterpret_cast<unsigned short*>(am.stage + 32 * 10);
   }
   const bool colors = cache_colors_on(p);
-  const bool sh16 = !p.cols && p.M == 16 && p.sh_degree == 3;
+  const bool sh16 = !p.cols && p.M == 16 && p.sh_degree == 3 && on_16_bytes(p.d_sh);
   const int row = p.cols ? 3 : 3 * sh_count(p.sh_degree);  // colour gradients of a hit
   unsigned replays = 0;
   Counters cnt;  // (interval continuations and re-traces are the forward's to count)

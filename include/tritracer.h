@@ -93,7 +93,8 @@ typedef struct tt_config {
 
 /* Arguments of the forward trace: OptixTracer::trace_fwd
  * (tritracer/tracer.h:78-95, tracer.cpp:16-142). All pointers are device
- * pointers except gpu_time_ms. */
+ * pointers except gpu_time_ms; float and int arrays may start at any element
+ * (SH rows go faster where they start on 16 bytes). */
 typedef struct tt_fwd_args {
   int H, W;
   const float* ray_o;
