@@ -2394,17 +2394,13 @@ __device__ __noinline__ void window_bwd_exact(const Geom& g, float3 dir, float d
   }
 }
 
-// Upstream gradients of one ray, and what its adjoint needs of the forward's
-// outputs. backward.cu:296-312 forms dL/dalpha per channel as
-// g (T x - (X_final - X) / (1 - alpha)), X the channel's running sum of w x
-// including the current hit; summed over the channels that is
-// T q - (F - S) / (1 - alpha) with q = sum g x, S = sum w q and F = sum g X_final:
-// one running sum instead of seven.
+// Upstream gradients of one ray and what its adjoint needs of the forward's
+// outputs.
 struct RayGrads {
   float g0, g1, g2, gD, gN0, gN1, gN2;
-  float F;
+  float Cf0, Cf1, Cf2, Df, Nf0, Nf1, Nf2;
   // EXACT: middepth / distortion
-  float Df, Wf, distf, gMid, gDist;
+  float Wf, distf, gMid, gDist;
 };
 
 template <bool EXACT>
@@ -2418,10 +2414,13 @@ __device__ __forceinline__ RayGrads load_ray_grads(const ViewDesc& v, int pix) {
   r.gN0 = __ldg(v.dL_doth + (kNormalCh + 0) * HW + pix);
   r.gN1 = __ldg(v.dL_doth + (kNormalCh + 1) * HW + pix);
   r.gN2 = __ldg(v.dL_doth + (kNormalCh + 2) * HW + pix);
+  r.Cf0 = __ldg(v.colors + pix);
+  r.Cf1 = __ldg(v.colors + HW + pix);
+  r.Cf2 = __ldg(v.colors + 2 * HW + pix);
   r.Df = __ldg(v.others + kDepthCh * HW + pix);
-  r.F = r.g0 * __ldg(v.colors + pix) + r.g1 * __ldg(v.colors + HW + pix) + r.g2 * __ldg(v.colors + 2 * HW + pix) +
-        r.gD * r.Df + r.gN0 * __ldg(v.others + (kNormalCh + 0) * HW + pix) +
-        r.gN1 * __ldg(v.others + (kNormalCh + 1) * HW + pix) + r.gN2 * __ldg(v.others + (kNormalCh + 2) * HW + pix);
+  r.Nf0 = __ldg(v.others + (kNormalCh + 0) * HW + pix);
+  r.Nf1 = __ldg(v.others + (kNormalCh + 1) * HW + pix);
+  r.Nf2 = __ldg(v.others + (kNormalCh + 2) * HW + pix);
   if (EXACT) {
     r.Wf = __ldg(v.others + kAlphaCh * HW + pix);
     r.distf = __ldg(v.others + kDistortionCh * HW + pix);
@@ -2429,6 +2428,30 @@ __device__ __forceinline__ RayGrads load_ray_grads(const ViewDesc& v, int pix) {
     r.gDist = __ldg(v.dL_doth + kDistortionCh * HW + pix);
   }
   return r;
+}
+
+// backward.cu:296-312 forms dL/dalpha per channel as
+// g (T x - (X_final - X) / (1 - alpha)), X the channel's running sum of w x up to
+// and with the current hit. Each X repeats the forward's additions in the forward's
+// order, so its rounding cancels against X_final's and the rest behind the hit is
+// as good as its own terms; one sum over the channels, or another order, leaves
+// that rounding in, multiplied by up to 100 (L2 error of dL/dalpha against FP64
+// 1.6 to 2.2 times as large).
+struct RaySums {
+  float C0 = 0.f, C1 = 0.f, C2 = 0.f, N0 = 0.f, N1 = 0.f, N2 = 0.f, D = 0.f;
+  __device__ __forceinline__ void add(float c0, float c1, float c2, float3 n, float t, float w) {
+    C0 += c0 * w;
+    C1 += c1 * w;
+    C2 += c2 * w;
+    N0 += n.x * w;
+    N1 += n.y * w;
+    N2 += n.z * w;
+    D += w * t;
+  }
+};
+__device__ __forceinline__ float alpha_grad_color(float g0, float g1, float g2, float c0, float c1, float c2, float b0,
+                                                  float b1, float b2, float T, float inv1a) {
+  return g0 * (T * c0 - b0 * inv1a) + g1 * (T * c1 - b1 * inv1a) + g2 * (T * c2 - b2 * inv1a);
 }
 
 // One blended hit's opacity and sigma gradients, scattered, and its vertex
@@ -2496,7 +2519,7 @@ __device__ __forceinline__ void scatter_hit(const TraceParams& p, uint32_t prim,
 }
 
 // backward.cu:191-350: the same march, dL/dalpha from the final values and the
-// running sum, scattered gradients. EXACT: the full chain rule of
+// running sums, scattered gradients. EXACT: the full chain rule of
 // window_bwd_exact, and no gradient through a clamped alpha.
 template <int MODE>
 struct BwdShader {
@@ -2509,7 +2532,8 @@ struct BwdShader {
   // upstream gradients and finals, loaded for each chunk (so they do not
   // occupy registers during traversal)
   RayGrads r;
-  float S, T;
+  RaySums x;
+  float T;
   float Sd;  // EXACT: running sum of the distortion's w E
   bool mid_seen;
 
@@ -2520,7 +2544,7 @@ struct BwdShader {
     pix = pixel;
     o = ro;
     d = rd;
-    S = 0.f;
+    x = RaySums{};
     T = 1.0f;
     Sd = 0.f;
     mid_seen = false;
@@ -2566,10 +2590,12 @@ struct BwdShader {
     }
     const float c0 = p.cols ? raw.x : fmaxf(raw.x, 0.f), c1 = p.cols ? raw.y : fmaxf(raw.y, 0.f),
                 c2 = p.cols ? raw.z : fmaxf(raw.z, 0.f);
-    const float q = r.g0 * c0 + r.g1 * c1 + r.g2 * c2 + r.gD * g.t + r.gN0 * g.n.x + r.gN1 * g.n.y + r.gN2 * g.n.z;
-    S += w * q;
+    x.add(c0, c1, c2, g.n, g.t, w);
     const float inv1a = 1.0f / (1.0f - alpha);
-    float dL_dalpha = T * q - (r.F - S) * inv1a;
+    float dL_dalpha = alpha_grad_color(r.g0, r.g1, r.g2, c0, c1, c2, r.Cf0 - x.C0, r.Cf1 - x.C1, r.Cf2 - x.C2, T, inv1a);
+    dL_dalpha += r.gD * (T * g.t - (r.Df - x.D) * inv1a);
+    dL_dalpha += alpha_grad_color(r.gN0, r.gN1, r.gN2, g.n.x, g.n.y, g.n.z, r.Nf0 - x.N0, r.Nf1 - x.N1, r.Nf2 - x.N2, T,
+                                  inv1a);
     float dL_dt = r.gD * w;
     if (EXACT) {
       // distortion: dD/dalpha_k = T_k E_k - (2 D_f - S_k) / (1 - alpha_k),
@@ -2614,14 +2640,15 @@ __global__ void __launch_bounds__(kTraceThreads, kMinBlocks) k_backward(const __
 // lanes at work on the benchmark's clouds, each step waiting on its gathers.
 // Here each ray's march only lists its next hits (kVisits a round); the lists
 // of the tile's rays are laid end to end and taken 32 at a time, and what a
-// hit needs of the ones before it on its ray, the transmittance and the sum
-// of w q, run along the ray's lanes and are carried from one step to the next
+// hit needs of the ones before it on its ray, the transmittance and the channels'
+// running sums, run along the ray's lanes and are carried from one step to the next
 // in shared memory. A ray ends at the first hit whose transmittance falls below
 // the cut-off; the transmittance is multiplied hit by hit, in the forward's
 // order, because a product that rounds differently ends a ray that lies on the
-// cut-off elsewhere than the forward did, where the cache holds no next query.
-// A ray has at most kVisits lanes of a step, so that chain is as short as the
-// scan of the sums.
+// cut-off elsewhere than the forward did, where the cache holds no next query. The
+// sums follow the forward hit by hit too (RaySums says why); depth and normals
+// are summed only where one of the tile's rays has a gradient there.
+// A ray has at most kVisits lanes of a step, so those chains are short.
 //
 // What bounds it then is L2's handling of the reductions: 23 a hit (12 of 16
 // bytes, the others of 4), each a request and a sector of its own when every
@@ -2634,8 +2661,12 @@ __global__ void __launch_bounds__(kTraceThreads, kMinBlocks) k_backward(const __
 // triangles, 4 views of 800^2, 28M blended hits 4.2 / 4.3 / 2.9; 3M triangles,
 // 16 views, 180M hits 39.0 / 38.6 / 20.5; exact adjoint of 200k triangles
 // 0.24 / 0.18 / 0.18. (Scans over the whole warp instead of a ray's lanes: 3.2 and
-// 22.1.) It issues on 46 % of cycles with L2 39 % and DRAM 16 %
-// busy: bound by instructions and their latency at 16 warps per SM.
+// 22.1.) These are with one sum over all channels; the channels' own sums made a step
+// of the 1M triangles 9.49 instead of 9.20 ms, of the exact 200k 0.59 instead of 0.57.
+// It issues on under half of the cycles, with L2 35 and DRAM 15 % busy: bound by
+// instructions and their latency at 16 warps per SM. Its loop is as long as the
+// instruction cache: waits for instructions doubled (0.7 to 1.6 of ~9 cycles an
+// instruction) with the sums' chain unrolled and the SH evaluation inlined, 9.76 ms a step.
 constexpr int kVisits = 6;
 
 // Inclusive sum over the lanes of a segment (first lane `seg`) of at most 8.
@@ -2649,16 +2680,28 @@ __device__ __forceinline__ float seg_sum(float v, int lane, int seg) {
   return v;
 }
 
+// (out of line: only an adjoint whose cache has no colours evaluates them)
+__device__ __noinline__ float3 sh_raw_cold(const float* shs, int M, int deg, int prim, const float* basis) {
+  float B[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) B[i] = basis[i];
+  return sh_raw(shs, M, prim, deg, B);
+}
 struct AdjointMem {
-  float4* ray;          // [4][32]: o, gD | d, F | g, T | gN, S (T < 0: the ray has ended)
-  float4* exact;        // [2][32] EXACT: Df, Wf, distf, gDist | gMid, Sd
+  // [4][32]: d, gD | g, T | N, D or Cf, o.x | C, gN0 (T < 0: the ray has ended); [32]: gN1, gN2 or o.y, o.z.
+  // A tile without gradients of depth and normals keeps its rays' colours and
+  // origins where their sums and gradients would lie; one with them reads both from
+  // memory (18 floats a ray are what leaves 4 blocks of 32-hit queries an SM).
+  float4* ray;
+  float2* gn12;
+  float* exact;         // [3][32] EXACT: gDist, gMid, Sd
   float* basis;         // [32][16] SH basis
   float* stage;         // [32][8] e0 e1 e2 e0 e1, prim, ray | [32][9] vertex gradients, [32] first vertex
   unsigned short* list; // [32 * kVisits]: ray << 8 | slot
 };
 template <int MODE>
 constexpr size_t adjoint_warp_bytes() {
-  return (size_t)32 * 16 * (4 + 4 + (MODE == kShadeExact ? 2 : 0)) + 32 * 10 * 4 + 32 * kVisits * 2;
+  return (size_t)32 * (16 * (4 + 4) + 8 + (MODE == kShadeExact ? 12 : 0)) + 32 * 10 * 4 + 32 * kVisits * 2;
 }
 template <int K, int MODE>
 constexpr size_t adjoint_smem() {
@@ -2684,10 +2727,11 @@ __global__ void __launch_bounds__(kTraceThreads, kAdjointBlocks) k_adjoint(const
   {
     unsigned char* base = smem_raw + (size_t)K * blockDim.x * 8 + (threadIdx.x >> 5) * adjoint_warp_bytes<MODE>();
     am.ray = reinterpret_cast<float4*>(base);
-    am.exact = am.ray + 4 * 32;
-    am.basis = reinterpret_cast<float*>(am.exact + (EXACT ? 2 * 32 : 0));
+    am.basis = reinterpret_cast<float*>(am.ray + 4 * 32);
     am.stage = am.basis + 16 * 32;
-    am.list = reinterpret_cast<unsigned short*>(am.stage + 32 * 10);
+    am.gn12 = reinterpret_cast<float2*>(am.stage + 32 * 10);
+    am.exact = reinterpret_cast<float*>(am.gn12 + 32);
+    am.list = reinterpret_cast<unsigned short*>(am.exact + (EXACT ? 3 * 32 : 0));
   }
   const bool colors = cache_colors_on(p);
   const bool sh16 = !p.cols && p.M == 16 && p.sh_degree == 3 && on_16_bytes(p.d_sh);
@@ -2705,22 +2749,29 @@ __global__ void __launch_bounds__(kTraceThreads, kAdjointBlocks) k_adjoint(const
     const int lt = tile - v.tile_begin;
     const int px = (lt % v.ntx) * 8 + (lane & 7), py = (lt / v.ntx) * 4 + (lane >> 3);
     bool active = px < v.W && py < v.H && (lane << p.parts_log) >> 5 == part;
+    const int pix0 = (lt / v.ntx) * 4 * v.W + (lt % v.ntx) * 8, HW = v.H * v.W;
+    bool other = false;  // the ray has a gradient of depth or normals
     Cursor cur = first_cursor(p.tmin_inclusive);
     long long ray_g = 0;
     if (active) {
       const int pix = py * v.W + px;
       ray_g = v.ray_begin + pix;
-      const float3 o = make_float3(v.ray_o[3 * pix], v.ray_o[3 * pix + 1], v.ray_o[3 * pix + 2]);
       const float3 d = make_float3(v.ray_d[3 * pix], v.ray_d[3 * pix + 1], v.ray_d[3 * pix + 2]);
-      if (v.interval) clip_cursor(cur, v.interval, v.H * v.W, pix);
-      const RayGrads r = load_ray_grads<EXACT>(v, pix);
-      am.ray[lane] = make_float4(o.x, o.y, o.z, r.gD);
-      am.ray[32 + lane] = make_float4(d.x, d.y, d.z, r.F);
-      am.ray[64 + lane] = make_float4(r.g0, r.g1, r.g2, 1.0f);
-      am.ray[96 + lane] = make_float4(r.gN0, r.gN1, r.gN2, 0.0f);
+      if (v.interval) clip_cursor(cur, v.interval, HW, pix);
+      const float gD = __ldg(v.dL_doth + kDepthCh * HW + pix);
+      const float gN0 = __ldg(v.dL_doth + (kNormalCh + 0) * HW + pix);
+      const float gN1 = __ldg(v.dL_doth + (kNormalCh + 1) * HW + pix);
+      const float gN2 = __ldg(v.dL_doth + (kNormalCh + 2) * HW + pix);
+      other = gD != 0.f || gN0 != 0.f || gN1 != 0.f || gN2 != 0.f;
+      am.ray[lane] = make_float4(d.x, d.y, d.z, gD);
+      am.ray[32 + lane] =
+          make_float4(__ldg(v.dL_dpix + pix), __ldg(v.dL_dpix + HW + pix), __ldg(v.dL_dpix + 2 * HW + pix), 1.0f);
+      am.ray[96 + lane] = make_float4(0.f, 0.f, 0.f, gN0);
+      am.gn12[lane] = make_float2(gN1, gN2);
       if (EXACT) {
-        am.exact[lane] = make_float4(r.Df, r.Wf, r.distf, r.gDist);
-        am.exact[32 + lane] = make_float4(r.gMid, 0.0f, 0.0f, 0.0f);
+        am.exact[lane] = __ldg(v.dL_doth + kDistortionCh * HW + pix);
+        am.exact[32 + lane] = __ldg(v.dL_doth + kMidDepthCh * HW + pix);
+        am.exact[64 + lane] = 0.0f;
       }
       if (!p.cols) {
         float B[16];
@@ -2731,6 +2782,15 @@ __global__ void __launch_bounds__(kTraceThreads, kAdjointBlocks) k_adjoint(const
         for (int i = 0; i < 4; ++i)
           reinterpret_cast<float4*>(am.basis + 16 * lane)[i] = make_float4(B[4 * i], B[4 * i + 1], B[4 * i + 2], B[4 * i + 3]);
       }
+    }
+    const bool others = __any_sync(full, other);
+    if (others) {
+      am.ray[64 + lane] = make_float4(0.f, 0.f, 0.f, 0.f);
+    } else if (active) {
+      const int pix = py * v.W + px;
+      am.ray[64 + lane] =
+          make_float4(__ldg(v.colors + pix), __ldg(v.colors + HW + pix), __ldg(v.colors + 2 * HW + pix), v.ray_o[3 * pix]);
+      am.gn12[lane] = make_float2(v.ray_o[3 * pix + 1], v.ray_o[3 * pix + 2]);
     }
     uint32_t next = kNoEntry;
     for (bool first = true; __any_sync(full, active); first = false) {
@@ -2792,10 +2852,9 @@ __global__ void __launch_bounds__(kTraceThreads, kAdjointBlocks) k_adjoint(const
           float* crow = reinterpret_cast<float*>(
               __shfl_sync(full, reinterpret_cast<unsigned long long>(rows), ray & 31));
           const int cstride = __shfl_sync(full, rstride, ray & 31);
-          float T0 = -1.0f, S0 = 0.f;
-          float4 q1, q2, q3;  // d, F | g, T | gN, S
-          float4 x0 = make_float4(0.f, 0.f, 0.f, 0.f), x1 = x0;
-          float gD = 0.f;
+          float T0 = -1.0f;
+          float4 q0, q1;  // d, gD | g, T
+          const int pix = pix0 + ((ray & 31) >> 3) * v.W + (ray & 7);  // the ray's
           Geom g;
           float alpha = 0.f, opacity = 0.f, sig = 0.f;
           uint32_t prim = 0;
@@ -2812,15 +2871,17 @@ __global__ void __launch_bounds__(kTraceThreads, kAdjointBlocks) k_adjoint(const
             else if (crow)
               raw = make_float3(crow[(size_t)slot * cstride], crow[(size_t)slot * cstride + 1],
                                 crow[(size_t)slot * cstride + 2]);
-            const float4 q0 = am.ray[ray];
+            float3 o;
+            if (others) {
+              o = make_float3(__ldg(v.ray_o + 3 * pix), __ldg(v.ray_o + 3 * pix + 1), __ldg(v.ray_o + 3 * pix + 2));
+            } else {
+              const float2 yz = am.gn12[ray];
+              o = make_float3(reinterpret_cast<const float*>(am.ray + 64 + ray)[3], yz.x, yz.y);
+            }
+            q0 = am.ray[ray];
             q1 = am.ray[32 + ray];
-            q2 = am.ray[64 + ray];
-            q3 = am.ray[96 + ray];
-            gD = q0.w;
-            T0 = q2.w;
-            S0 = q3.w;
-            if (EXACT) x1 = am.exact[32 + ray];  // gMid, Sd
-            g = shade_geom<MODE>(a, b, c, make_float3(q0.x, q0.y, q0.z), make_float3(q1.x, q1.y, q1.z), key_t(key), sig);
+            T0 = q1.w;
+            g = shade_geom<MODE>(a, b, c, o, make_float3(q0.x, q0.y, q0.z), key_t(key), sig);
             alpha = fminf(kAlphaMax, opacity * g.Cx);
             if (alpha < kAlphaMin) alpha = 0.f;
           }
@@ -2838,43 +2899,90 @@ __global__ void __launch_bounds__(kTraceThreads, kAdjointBlocks) k_adjoint(const
           const bool dead = (ended & (full << seg) & (full >> (31 - lane))) != 0u;
           const bool blend = on && alpha > 0.f && !dead;
           const float w = blend ? alpha * T : 0.f;
-          float q = 0.f, E = 0.f;
+          float c0 = 0.f, c1 = 0.f, c2 = 0.f, E = 0.f;
+          float Cf0, Cf1, Cf2;                    // the ray's outputs
+          float Df = 0.f, Wf = 0.f, distf = 0.f;  // EXACT
+          float4 x = make_float4(0.f, 0.f, 0.f, 0.f);  // running sums of the colour, gN0
+          if (on) x = am.ray[96 + ray];
           if (blend) {
-            if (!p.cols && !crow) {
-              float B[16];
-#pragma unroll
-              for (int i = 0; i < 16; ++i) B[i] = am.basis[16 * ray + i];
-              raw = sh_raw(p.shs, p.M, (int)prim, p.sh_degree, B);
+            if (others) {
+              Cf0 = __ldg(v.colors + pix);
+              Cf1 = __ldg(v.colors + HW + pix);
+              Cf2 = __ldg(v.colors + 2 * HW + pix);
+            } else {
+              const float4 y = am.ray[64 + ray];
+              Cf0 = y.x;
+              Cf1 = y.y;
+              Cf2 = y.z;
             }
-            const float c0 = p.cols ? raw.x : fmaxf(raw.x, 0.f), c1 = p.cols ? raw.y : fmaxf(raw.y, 0.f),
-                        c2 = p.cols ? raw.z : fmaxf(raw.z, 0.f);
-            q = q2.x * c0 + q2.y * c1 + q2.z * c2 + gD * g.t + q3.x * g.n.x + q3.y * g.n.y + q3.z * g.n.z;
+            if (!p.cols && !crow) raw = sh_raw_cold(p.shs, p.M, p.sh_degree, (int)prim, am.basis + 16 * ray);
+            c0 = p.cols ? raw.x : fmaxf(raw.x, 0.f);
+            c1 = p.cols ? raw.y : fmaxf(raw.y, 0.f);
+            c2 = p.cols ? raw.z : fmaxf(raw.z, 0.f);
             if (EXACT) {
-              x0 = am.exact[ray];  // Df, Wf, distf, gDist
-              const float Cf = x0.y > 0.f ? (x0.z + x0.x * x0.x) / x0.y : 0.f;
-              E = g.t * g.t * x0.y - 2.0f * g.t * x0.x + Cf;
+              Df = __ldg(v.others + kDepthCh * HW + pix);
+              Wf = __ldg(v.others + kAlphaCh * HW + pix);
+              distf = __ldg(v.others + kDistortionCh * HW + pix);
+              const float Cf = Wf > 0.f ? (distf + Df * Df) / Wf : 0.f;
+              E = g.t * g.t * Wf - 2.0f * g.t * Df + Cf;
             }
           }
-          const float S = S0 + seg_sum(w * q, lane, seg);
+          // the running sums, hit by hit like the transmittance
+          const float w0 = c0 * w, w1 = c1 * w, w2 = c2 * w;
+          x.x += w0, x.y += w1, x.z += w2;
+#pragma unroll 1  // (unrolled, the kernel's code passes the instruction cache)
+          for (int i = 1; i < kVisits; ++i) {
+            const float u0 = __shfl_up_sync(full, x.x, 1), u1 = __shfl_up_sync(full, x.y, 1),
+                        u2 = __shfl_up_sync(full, x.z, 1);
+            if (lane - seg == i) x.x = u0 + w0, x.y = u1 + w1, x.z = u2 + w2;
+          }
           float Sd = 0.f;
-          if (EXACT) Sd = x1.y + seg_sum(w * E, lane, seg);
+          if (EXACT) Sd = (on ? am.exact[64 + ray] : 0.f) + seg_sum(w * E, lane, seg);
+          const float inv1a = 1.0f / (1.0f - alpha);
+          float dL_dalpha = 0.f;
+          if (blend)
+            dL_dalpha = alpha_grad_color(q1.x, q1.y, q1.z, c0, c1, c2, Cf0 - x.x, Cf1 - x.y, Cf2 - x.z, T, inv1a);
+          float3 dL_dn = make_float3(0.f, 0.f, 0.f);
+          if (others) {
+            float4 y = on ? am.ray[64 + ray] : make_float4(0.f, 0.f, 0.f, 0.f);
+            const float n0 = blend ? g.n.x * w : 0.f, n1 = blend ? g.n.y * w : 0.f, n2 = blend ? g.n.z * w : 0.f,
+                        nD = blend ? w * g.t : 0.f;
+            y.x += n0, y.y += n1, y.z += n2, y.w += nD;
+#pragma unroll 1
+            for (int i = 1; i < kVisits; ++i) {
+              const float u0 = __shfl_up_sync(full, y.x, 1), u1 = __shfl_up_sync(full, y.y, 1),
+                          u2 = __shfl_up_sync(full, y.z, 1), uD = __shfl_up_sync(full, y.w, 1);
+              if (lane - seg == i) y.x = u0 + n0, y.y = u1 + n1, y.z = u2 + n2, y.w = uD + nD;
+            }
+            if (blend) {
+              const float2 gn = am.gn12[ray];
+              dL_dn = make_float3(x.w * w, gn.x * w, gn.y * w);
+              const float D = EXACT ? Df : __ldg(v.others + kDepthCh * HW + pix);
+              const float Nf0 = __ldg(v.others + (kNormalCh + 0) * HW + pix);
+              const float Nf1 = __ldg(v.others + (kNormalCh + 1) * HW + pix);
+              const float Nf2 = __ldg(v.others + (kNormalCh + 2) * HW + pix);
+              dL_dalpha += q0.w * (T * g.t - (D - y.w) * inv1a);
+              dL_dalpha += alpha_grad_color(x.w, gn.x, gn.y, g.n.x, g.n.y, g.n.z, Nf0 - y.x, Nf1 - y.y, Nf2 - y.z, T, inv1a);
+            }
+            __syncwarp();
+            if (tail) am.ray[64 + ray] = y;
+          }
           const unsigned bm = __ballot_sync(full, blend);
           const int nb = __popc(bm), rank = __popc(bm & ((1u << lane) - 1u));
           float3 gv[3];
           if (blend) {
-            const float inv1a = 1.0f / (1.0f - alpha);
-            float dL_dalpha = T * q - (q1.w - S) * inv1a;
-            float dL_dt = gD * w;
+            float dL_dt = q0.w * w;
             if (EXACT) {
-              dL_dalpha += x0.w * (T * E - (2.0f * x0.z - Sd) * inv1a);
-              dL_dt += x0.w * 2.0f * w * (g.t * x0.y - x0.x);
-              if (T > 0.5f && test_T <= 0.5f) dL_dt += x1.x;
+              const float gDist = am.exact[ray];
+              dL_dalpha += gDist * (T * E - (2.0f * distf - Sd) * inv1a);
+              dL_dt += gDist * 2.0f * w * (g.t * Wf - Df);
+              if (T > 0.5f && test_T <= 0.5f) dL_dt += am.exact[32 + ray];
             }
-            hit_grads<MODE>(p, prim, g, make_float3(q1.x, q1.y, q1.z), sig, opacity, dL_dalpha, dL_dt,
-                            make_float3(q3.x * w, q3.y * w, q3.z * w), gv);
+            hit_grads<MODE>(p, prim, g, make_float3(q0.x, q0.y, q0.z), sig, opacity, dL_dalpha, dL_dt,
+                            dL_dn, gv);
             // colour gradients: dRGB/dsh_k = B_k, masked where the colour was clamped at 0
             const bool m0 = !p.cols && raw.x < 0.f, m1 = !p.cols && raw.y < 0.f, m2 = !p.cols && raw.z < 0.f;
-            const float e0 = m0 ? 0.f : q2.x * w, e1 = m1 ? 0.f : q2.y * w, e2 = m2 ? 0.f : q2.z * w;
+            const float e0 = m0 ? 0.f : q1.x * w, e1 = m1 ? 0.f : q1.y * w, e2 = m2 ? 0.f : q1.z * w;
             float4* st = reinterpret_cast<float4*>(am.stage) + 2 * rank;
             st[0] = make_float4(e0, e1, e2, e0);
             st[1] = make_float4(e1, __uint_as_float(prim), __int_as_float(ray), 0.f);
@@ -2921,14 +3029,14 @@ __global__ void __launch_bounds__(kTraceThreads, kAdjointBlocks) k_adjoint(const
           }
           __syncwarp();
           if (tail) {
-            reinterpret_cast<float*>(am.ray + 64 + ray)[3] = dead ? -1.0f : test_T;
-            reinterpret_cast<float*>(am.ray + 96 + ray)[3] = S;
-            if (EXACT) reinterpret_cast<float*>(am.exact + 32 + ray)[1] = Sd;
+            reinterpret_cast<float*>(am.ray + 32 + ray)[3] = dead ? -1.0f : test_T;
+            am.ray[96 + ray] = x;
+            if (EXACT) am.exact[64 + ray] = Sd;
           }
           __syncwarp();
         }
         if (marching || active) {
-          if (reinterpret_cast<const float*>(am.ray + 64 + lane)[3] < 0.f) marching = active = false;
+          if (reinterpret_cast<const float*>(am.ray + 32 + lane)[3] < 0.f) marching = active = false;
         }
       }
     }
@@ -3502,8 +3610,10 @@ struct SecBwdShader {
   const ViewDesc* v;
   int ridx, pix, level;
   float3 o, d;
+  float Cf0, Cf1, Cf2, Df, Nf0, Nf1, Nf2;  // finals and upstream gradients as in RayGrads
   float g0, g1, g2, gD, gN0, gN1, gN2;
-  float F, S, T;  // as RayGrads::F and the running sum beside it
+  RaySums x;
+  float T;
   bool spawned;
 
   __device__ explicit SecBwdShader(const TraceParams& params) : p(params), v(&params.views[0]) {}
@@ -3534,22 +3644,26 @@ struct SecBwdShader {
       gN0 = __ldg(v->dL_doth + (kNormalCh + 0) * HW + pix);
       gN1 = __ldg(v->dL_doth + (kNormalCh + 1) * HW + pix);
       gN2 = __ldg(v->dL_doth + (kNormalCh + 2) * HW + pix);
-      F = gD * __ldg(v->others + kDepthCh * HW + pix) + gN0 * __ldg(v->others + (kNormalCh + 0) * HW + pix) +
-          gN1 * __ldg(v->others + (kNormalCh + 1) * HW + pix) + gN2 * __ldg(v->others + (kNormalCh + 2) * HW + pix);
+      Df = __ldg(v->others + kDepthCh * HW + pix);
+      Nf0 = __ldg(v->others + (kNormalCh + 0) * HW + pix);
+      Nf1 = __ldg(v->others + (kNormalCh + 1) * HW + pix);
+      Nf2 = __ldg(v->others + (kNormalCh + 2) * HW + pix);
     } else {
       ro = make_float3(r->o[0], r->o[1], r->o[2]);
       rd = make_float3(r->d[0], r->d[1], r->d[2]);
       pix = r->pixel;
       tau = r->tau;
-      F = gD = gN0 = gN1 = gN2 = 0.f;
+      Df = Nf0 = Nf1 = Nf2 = gD = gN0 = gN1 = gN2 = 0.f;
     }
     g0 = tau * __ldg(v->dL_dpix + pix);
     g1 = tau * __ldg(v->dL_dpix + HW + pix);
     g2 = tau * __ldg(v->dL_dpix + 2 * HW + pix);
-    F += g0 * r->L[0] + g1 * r->L[1] + g2 * r->L[2];
+    Cf0 = r->L[0];
+    Cf1 = r->L[1];
+    Cf2 = r->L[2];
     o = ro;
     d = rd;
-    S = 0.f;
+    x = RaySums{};
     T = 1.0f;
     spawned = false;
   }
@@ -3602,9 +3716,13 @@ struct SecBwdShader {
       c1 = fmaxf(raw.y, 0.f);
       c2 = fmaxf(raw.z, 0.f);
     }
-    const float q = g0 * c0 + g1 * c1 + g2 * c2 + gD * g.t + gN0 * g.n.x + gN1 * g.n.y + gN2 * g.n.z;
-    S += w * q;
-    const float dL_dalpha = T * q - (F - S) * (1.0f / (1.0f - alpha));
+    x.add(c0, c1, c2, g.n, g.t, w);
+    const float inv1a = 1.0f / (1.0f - alpha);
+    float dL_dalpha = alpha_grad_color(g0, g1, g2, c0, c1, c2, Cf0 - x.C0, Cf1 - x.C1, Cf2 - x.C2, T, inv1a);
+    if (level == 0) {  // spawned rays only pass colour on
+      dL_dalpha += gD * (T * g.t - (Df - x.D) * inv1a);
+      dL_dalpha += alpha_grad_color(gN0, gN1, gN2, g.n.x, g.n.y, g.n.z, Nf0 - x.N0, Nf1 - x.N1, Nf2 - x.N2, T, inv1a);
+    }
     const float3 dL_dn = make_float3(gN0 * w, gN1 * w, gN2 * w);
     float3 gv[3];
     if (p.mode == kShadeExact)  // the full chain rule of the window function and the face normal; spawn geometry held constant
