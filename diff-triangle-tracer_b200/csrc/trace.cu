@@ -283,9 +283,11 @@ __device__ __forceinline__ void query(const BvhView& bvh, const RayW& r, unsigne
 // two lines u = off + slope z', and so does its v. Rays of one origin have the
 // lines of their extreme slopes; for others the chords between the extreme
 // positions at z0 and z1 bound them (the maximum of linear functions is
-// convex). Everything is padded by 2^-17 of the largest coordinate involved,
-// an order above the rounding of these lines (slopes are at most 2) and of the
-// watertight test itself.
+// convex). Everything is padded by 2^-17 of the largest coordinate inside the
+// frustum, an order above the rounding of these lines (slopes are at most 2) and of
+// boxes clipped to it. A triangle's vertices may lie far outside: the cull and the
+// watertight test shear each of them, with some ten roundings of 2^-24 of its own
+// coordinates, so a triangle is culled only beyond 2^-20 of its largest.
 //
 // A wide frustum (coarse images, unrelated rays) holds many more triangles
 // than its rays hit. Such a warp takes its rays one by one: the frustum is
@@ -305,6 +307,7 @@ constexpr int kWarpRoom = 80;    // entries after a wave of several nodes: 56 ar
 constexpr int kWarpQueue = 128;  // triangles of entered leaves (ring)
 constexpr int kWarpKept = 64;    // triangles the frustum kept (ring)
 constexpr int kWarpPairs = 64;   // (triangle, ray) pairs tested between two compactions
+constexpr float kVertexMargin = 9.5367431640625e-7f;
 constexpr int kSpare = 4;        // slots of a ray's buffer beyond its K keys
 
 struct WarpStack {
@@ -651,11 +654,15 @@ __device__ __forceinline__ void packet_query(const BvhView& bvh, const RayW& r, 
           const float Au = sel3(A.y, A.z, A.x, kz), Av = sel3(A.z, A.x, A.y, kz), Az = sg * sel3(A.x, A.y, A.z, kz);
           const float Bu = sel3(B.y, B.z, B.x, kz), Bv = sel3(B.z, B.x, B.y, kz), Bz = sg * sel3(B.x, B.y, B.z, kz);
           const float Cu = sel3(C.y, C.z, C.x, kz), Cv = sel3(C.z, C.x, C.y, kz), Cz = sg * sel3(C.x, C.y, C.z, kz);
-          keep = (max3f(Az, Bz, Cz) >= z0) & (min3f(Az, Bz, Cz) <= zcur) &
-                 (min3f(fmaf(-sU1, Az, Au), fmaf(-sU1, Bz, Bu), fmaf(-sU1, Cz, Cu)) <= oU1) &
-                 (max3f(fmaf(-sU0, Az, Au), fmaf(-sU0, Bz, Bu), fmaf(-sU0, Cz, Cu)) >= oU0) &
-                 (min3f(fmaf(-sV1, Az, Av), fmaf(-sV1, Bz, Bv), fmaf(-sV1, Cz, Cv)) <= oV1) &
-                 (max3f(fmaf(-sV0, Az, Av), fmaf(-sV0, Bz, Bv), fmaf(-sV0, Cz, Cv)) >= oV0);
+          // pad covers what lies in the frustum; a vertex outside it rounds by its own size
+          const float e = kVertexMargin * max3f(max3f(fabsf(Au), fabsf(Bu), fabsf(Cu)),
+                                                max3f(fabsf(Av), fabsf(Bv), fabsf(Cv)),
+                                                max3f(fabsf(Az), fabsf(Bz), fabsf(Cz)));
+          keep = (max3f(Az, Bz, Cz) >= z0 - e) & (min3f(Az, Bz, Cz) <= zcur + e) &
+                 (min3f(fmaf(-sU1, Az, Au), fmaf(-sU1, Bz, Bu), fmaf(-sU1, Cz, Cu)) <= oU1 + e) &
+                 (max3f(fmaf(-sU0, Az, Au), fmaf(-sU0, Bz, Bu), fmaf(-sU0, Cz, Cu)) >= oU0 - e) &
+                 (min3f(fmaf(-sV1, Az, Av), fmaf(-sV1, Bz, Bv), fmaf(-sV1, Cz, Cv)) <= oV1 + e) &
+                 (max3f(fmaf(-sV0, Az, Av), fmaf(-sV0, Bz, Bv), fmaf(-sV0, Cz, Cv)) >= oV0 - e);
         }
         const unsigned km = __ballot_sync(full, keep);
         if (keep) ws.kept[(kh + kn + __popc(km & lt)) & (kWarpKept - 1)] = ti;
