@@ -665,7 +665,8 @@ __device__ __forceinline__ void packet_query(const BvhView& bvh, const RayW& r, 
                  (max3f(fmaf(-sV0, Az, Av), fmaf(-sV0, Bz, Bv), fmaf(-sV0, Cz, Cv)) >= oV0 - e);
         }
         const unsigned km = __ballot_sync(full, keep);
-        if (keep) ws.kept[(kh + kn + __popc(km & lt)) & (kWarpKept - 1)] = ti;
+        if (keep && TT_IN_BOUNDS(status, kn + __popc(km) <= kWarpKept))
+          ws.kept[(kh + kn + __popc(km & lt)) & (kWarpKept - 1)] = ti;
         kn += __popc(km);
         __syncwarp();
         continue;
@@ -715,7 +716,7 @@ __device__ __forceinline__ void packet_query(const BvhView& bvh, const RayW& r, 
       if (b0 | b1) {
         const int at = qh + qn + __popc(b0 & lt) + 2 * __popc(b1 & lt);
         const uint32_t first = leaf_first(cref);
-        if (leaf) {
+        if (leaf && TT_IN_BOUNDS(status, at + (int)cnt - qh <= kWarpQueue)) {
           const bool ok = TT_IN_BOUNDS(status, first + cnt <= (uint32_t)bvh.P);
           ws.queue[at & (kWarpQueue - 1)] = ok ? first : 0u;
           if (cnt > 1u) ws.queue[(at + 1) & (kWarpQueue - 1)] = ok ? first + 1u : 0u;
@@ -737,7 +738,7 @@ __device__ __forceinline__ void packet_query(const BvhView& bvh, const RayW& r, 
           single = true;
           break;
         }
-        if (inner && rank < npush) {
+        if (inner && rank < npush && TT_IN_BOUNDS(status, sp >= 0 && sp + npush <= kWarpStack)) {
           ws.ref[sp + npush - 1 - rank] = cref;
           ws.z[sp + npush - 1 - rank] = (unsigned short)(__float_as_uint(za - z0) >> 16);
         }
@@ -880,6 +881,7 @@ __device__ __forceinline__ void pair_query(const BvhView& bvh, const RayW& r, bo
       more += __popc(inner[c]);
       if (h && leaf) {
         const uint32_t first = leaf_first(cref[c]), n = leaf_count(cref[c]);
+        if (!TT_IN_BOUNDS(status, at + (int)n - qh <= kPairQueue)) continue;
         const uint32_t f = ((TT_IN_BOUNDS(status, first + n <= (uint32_t)bvh.P) ? first : 0u) << 5) | (uint32_t)ray;
         pm.queue[at & (kPairQueue - 1)] = f;
         if (n > 1u) pm.queue[(at + 1) & (kPairQueue - 1)] = f + 32u;
@@ -892,7 +894,8 @@ __device__ __forceinline__ void pair_query(const BvhView& bvh, const RayW& r, bo
     if (sp + more <= kPairStack) {
 #pragma unroll
       for (int c = 0; c < 8; ++c) {
-        if ((inner[c] >> lane) & 1u) pm.stack[sp + __popc(inner[c] & lt)] = (cref[c] << 5) | (uint32_t)ray;
+        if (((inner[c] >> lane) & 1u) && TT_IN_BOUNDS(status, sp >= 0 && sp + __popc(inner[c]) <= kPairStack))
+          pm.stack[sp + __popc(inner[c] & lt)] = (cref[c] << 5) | (uint32_t)ray;
         sp += __popc(inner[c]);
       }
     } else {
@@ -2844,7 +2847,7 @@ __global__ void __launch_bounds__(kTraceThreads, kAdjointBlocks) k_adjoint(const
         }
         const int total = __shfl_sync(full, at, 31);
         at -= count;
-        for (int i = 0; i < count; ++i)
+        for (int i = 0; i < count && TT_IN_BOUNDS(p.status, at + i < 32 * kVisits); ++i)
           am.list[at + i] = (unsigned short)((lane << 8) | (int)((slots >> (8 * i)) & 0xFFu));
         __syncwarp();
         // ---- the hits of all rays, 32 at a time
@@ -2866,7 +2869,7 @@ __global__ void __launch_bounds__(kTraceThreads, kAdjointBlocks) k_adjoint(const
           float alpha = 0.f, opacity = 0.f, sig = 0.f;
           uint32_t prim = 0;
           float3 raw = make_float3(0.f, 0.f, 0.f);
-          if (on) {
+          if (on && TT_IN_BOUNDS(p.status, slot < K && ray < 32)) {
             const unsigned long long key = sm.keys[slot * sm.stride + (ray - lane)];
             prim = key_prim(key);
             const float4* tr = p.bvh.tri_prim + 3 * (size_t)prim;
