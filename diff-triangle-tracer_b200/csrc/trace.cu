@@ -361,11 +361,25 @@ __device__ __forceinline__ void warp_scene(const BvhView& bvh, const WarpStack& 
   __syncwarp();
 }
 
-// A packet is taken when the triangles its frustum holds number at most
-// kPacketMin + kPacketRatio times those its rays meet. Forwards of pinhole
-// images (ms; as packets / ray by ray): 1M triangles 128^2 3.5 / 5.8, 256^2
-// 1.7 / 5.7; 3M triangles 64^2 22.0 / 9.2, 128^2 8.5 / 9.3, 256^2 3.9 / 9.8;
-// 616k triangles 31 x 38 21.2 / 3.5; 100k triangles 64^2 0.6 / 1.0.
+// A packet is taken when the triangles its frustum holds are expected to number
+// at most kPacketMin + kPacketRatio times those its rays meet, for triangles of the
+// mean extent spread evenly over the scene's box. Forwards of pinhole images, every
+// warp with whole tiles (ms; as packets / ray by ray): 1M triangles 128^2 3.5 / 5.8,
+// 256^2 1.7 / 5.7; 3M triangles 64^2 22.0 / 9.2, 128^2 8.5 / 9.3, 256^2 3.9 / 9.8;
+// 616k triangles 31 x 38 21.2 / 3.5; 100k triangles 64^2 0.6 / 1.0. (Images as coarse
+// as the 64^2 and 31 x 38 are now taken in parts, a ray or two a warp.)
+//
+// One far triangle makes the box, and with it the expected spread, as large as
+// one likes. So the walk counts what its frustum does hold, and a packet past the
+// same line is given up for its rays: at once where the rays have no common origin,
+// as each triangle held then costs a test with every ray, and kPacketTrial times later where
+// a cull by the rays' lines makes it cheap. 65k rays in a cone from scattered origins over 200k
+// triangles, one of them 50 away: 278 ms without the count, 6.7 with it (8.5, 11.6 and
+// 17.3 at 2, 4 and 8 times the line; a walk with a box test per ray and child took 7.0).
+// A camera inside those triangles and a shell around them, 256^2 at 90 degrees: 5.2 ms
+// given up at the line, 4.4 at twice, 4.0 at 4 times. The count costs
+// 0.2 to 0.5 % (3M triangles at 1080p 7.76 / 7.80 ms).
+constexpr int kPacketTrial = 4, kPacketUnits = 2, kPacketMost = 1 << 30;
 constexpr float kPacketMin = 1024.0f, kPacketRatio = 2.5f;
 
 // Sorts the first n keys of a lane's column, of which the first `done` are in
@@ -387,12 +401,12 @@ __device__ __forceinline__ void kb_sort(unsigned long long* kb, int stride, int 
 // with that lane's ray, a hit appended to that lane's buffer. When a buffer has
 // no room, all are sorted and cut back to their K nearest, which bound their
 // rays' tmax, and what did not fit tries again if still near enough: returns
-// true then. `hits`: keys in each lane's buffer; kb_n: how many of this lane's
+// true then. `room` gains `gain` for each pair that meets, near or far. `hits`: keys in each lane's buffer; kb_n: how many of this lane's
 // are in order.
 template <int K>
 __device__ __forceinline__ bool test_pairs(const RayW& r, unsigned long long key_min, float& tmax, int& kb_n,
                                            unsigned long long* kb, int kstride, int* hits, bool have, int ray, float4 a,
-                                           float4 b, float4 c) {
+                                           float4 b, float4 c, int gain, int& room) {
   const unsigned full = 0xFFFFFFFFu;
   const int lane = threadIdx.x & 31;
   RayW q;
@@ -402,13 +416,13 @@ __device__ __forceinline__ bool test_pairs(const RayW& r, unsigned long long key
   const unsigned long long lo = __shfl_sync(full, key_min, ray);
   const float far = __shfl_sync(full, tmax, ray);
   unsigned long long key = kEmptyKey;
-  if (have) {
-    float t;
-    if (isect_tri_p(q, PermRt(q.perm), a, b, c, t) && t >= 0.f && t <= far) {
-      key = hit_key(t, (uint32_t)__float_as_int(a.w));
-      if (key < lo) key = kEmptyKey;
-    }
+  float t = 0.f;
+  const bool meets = have && isect_tri_p(q, PermRt(q.perm), a, b, c, t);
+  if (meets && t >= 0.f && t <= far) {
+    key = hit_key(t, (uint32_t)__float_as_int(a.w));
+    if (key < lo) key = kEmptyKey;
   }
+  if (gain != 0) room = min(room + gain * __popc(__ballot_sync(full, meets)), kPacketMost);
   bool cut = false;
   while (__any_sync(full, key != kEmptyKey)) {
     if (key != kEmptyKey) {
@@ -549,7 +563,7 @@ __device__ __forceinline__ void packet_query(const BvhView& bvh, const RayW& r, 
                          max3f(fabsf(fmaf(sV1, z1, oV1)), fabsf(fmaf(sV0, z1, oV0)), fabsf(fmaf(sV1, z0, oV1)))));
       pad = m * 7.62939453125e-6f;
       if (!single) {
-        // triangles the frustum holds against those its rays meet, for
+        // the expected triangles the frustum holds against those its rays meet, for
         // triangles of the mean extent spread over the scene's box
         const float zm = 0.5f * (z0 + z1);
         const float w = fmaf(sU1 - sU0, zm, oU1 - oU0), h = fmaf(sV1 - sV0, zm, oV1 - oV0);
@@ -577,6 +591,8 @@ __device__ __forceinline__ void packet_query(const BvhView& bvh, const RayW& r, 
     }
     __syncwarp();
     int sp = z0 <= z1 ? 1 : 0, qh = 0, qn = 0, kh = 0, kn = 0;
+    // triangles the frustum may still hold, in units of 1 / kPacketUnits of one
+    int room = (int)(kPacketMin * kPacketUnits) * (common ? kPacketTrial : 1);
     for (int steps = 0;; ++steps) {
       if (steps > kMaxSteps) {
         if (lane == 0) atomicOr(status, kStatusTimeout);
@@ -620,6 +636,7 @@ __device__ __forceinline__ void packet_query(const BvhView& bvh, const RayW& r, 
             if (lane >= i) at += v;
           }
           const int pairs = min(__shfl_sync(full, at, 31), kWarpPairs);
+          if (common) room = min(room + (int)(kPacketRatio * kPacketUnits) * kPacketTrial * pairs, kPacketMost);
           for (at -= __popc(m); m != 0u && at < kWarpPairs; ++at, m &= m - 1u)
             ws.pair[at] = (unsigned short)((lane << 5) | (__ffs(m) - 1));
           __syncwarp();
@@ -633,12 +650,18 @@ __device__ __forceinline__ void packet_query(const BvhView& bvh, const RayW& r, 
             c.x = __shfl_sync(full, C.x, tri), c.y = __shfl_sync(full, C.y, tri), c.z = __shfl_sync(full, C.z, tri);
             a.w = __shfl_sync(full, A.w, tri);
             b.w = c.w = 0.f;
-            if (test_pairs<K>(r, key_min, tmax, kb_n, kb, kstride, ws.hits, have, ray, a, b, c))
+            if (test_pairs<K>(r, key_min, tmax, kb_n, kb, kstride, ws.hits, have, ray, a, b, c,
+                              common ? 0 : (int)(kPacketRatio * kPacketUnits), room))
               zcur = fminf(z1, warp_max(in ? fmaf(tmax, dk, oz) : -INFINITY) + pad);
           }
           __syncwarp();
         }
         __syncwarp();
+        room -= n * kPacketUnits;
+        if (room < 0 && __popc(G) > 1) {
+          single = true;
+          break;
+        }
         continue;
       }
       if (qn >= 32 || (sp == 0 && qn > 0)) {
@@ -828,7 +851,8 @@ __device__ __forceinline__ void pair_query(const BvhView& bvh, const RayW& r, bo
       const float4* tr = bvh.tris + 3 * (size_t)(e >> 5);
       const float4 a = __ldg(tr), b = __ldg(tr + 1), c = __ldg(tr + 2);
       if (count_work && lane < n) ++cnt.tris;
-      test_pairs<K>(r, key_min, tmax, kb_n, kb, kstride, pm.hits, lane < n, (int)(e & 31u), a, b, c);
+      int room;
+      test_pairs<K>(r, key_min, tmax, kb_n, kb, kstride, pm.hits, lane < n, (int)(e & 31u), a, b, c, 0, room);
       __syncwarp();
       continue;
     }
