@@ -435,6 +435,10 @@ static int forward_impl(tt_tracer* h, const tt_fwd_args* a, const tt_view* views
                          (p.cfg == tt::kCfgPackets16 || p.cfg == tt::kCfgPackets32) ? 1 : 0;
     if (p.fwd_pair) ++h->trace_launches;
   }
+  if (tt::variant_may_go_by_lanes(p)) {  // two kernels, one of which works
+    p.fwd_pair = 1;
+    ++h->trace_launches;
+  }
   if (a->debug) TT_CUDA(h, cudaEventRecord(h->ev_mid, s));
   ++p.work;
   TT_CUDA(h, tt::launch_forward(p, h->fwd_grid, s));

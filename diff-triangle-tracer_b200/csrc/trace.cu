@@ -45,7 +45,7 @@ constexpr int kMinBlocks = TT_MIN_BLOCKS;
 // Per-lane traversal stack: the top SD entries in shared memory (strided by
 // the block size, conflict-free), continued in thread-local memory for deep
 // trees (only touched when the shared part is full).
-constexpr int kSpill = 64;
+constexpr int kLaneStack = 96;
 struct Stack {
   uint32_t* ref;
   float* tn;
@@ -176,6 +176,7 @@ __device__ __forceinline__ void query(const BvhView& bvh, const RayW& r, unsigne
   // word offsets of the near / far planes (lo at +0, hi at +2 within each axis)
   const int nx = r.ix >= 0.f ? 0 : 2, ny = r.iy >= 0.f ? 4 : 6, nz = r.iz >= 0.f ? 8 : 10;
   // entries at index >= SD live in thread-local memory
+  constexpr int kSpill = kLaneStack - SD;
   uint32_t xref[kSpill];
   float xtn[kSpill];
   auto put = [&](int i, uint32_t r, float t) {
@@ -337,19 +338,19 @@ __device__ __forceinline__ float warp_max(float v) {
   return r;
 }
 
-// Once per warp: the scene's box and the mean extent of 32 sampled triangles,
-// for the rule that decides between a packet and single rays.
-__device__ __forceinline__ void warp_scene(const BvhView& bvh, const WarpStack& ws) {
-  if (!bvh.has_root) return;
+// The scene's box and the mean extent of 32 sampled triangles, taken by a warp
+// for the rules that decide how rays are traversed.
+struct SceneStats {
+  float lo[3], hi[3], extent;
+};
+__device__ __forceinline__ SceneStats scene_stats(const BvhView& bvh) {
   const int lane = threadIdx.x & 31;
+  SceneStats st;
   const float* nd = reinterpret_cast<const float*>(bvh.nodes) + (lane & 7);
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
-    const float lo = warp_min(__ldg(nd + 16 * a)), hi = warp_max(__ldg(nd + 16 * a + 8));
-    if (lane == 0) {
-      ws.scene[a] = lo;
-      ws.scene[3 + a] = hi;
-    }
+    st.lo[a] = warp_min(__ldg(nd + 16 * a));
+    st.hi[a] = warp_max(__ldg(nd + 16 * a + 8));
   }
   const float4* tr = bvh.tris + 3 * (size_t)(((long long)lane * bvh.P) >> 5);
   const float4 a = __ldg(tr), b = __ldg(tr + 1), c = __ldg(tr + 2);
@@ -357,7 +358,21 @@ __device__ __forceinline__ void warp_scene(const BvhView& bvh, const WarpStack& 
             max3f(a.z, b.z, c.z) - min3f(a.z, b.z, c.z);
 #pragma unroll
   for (int s = 16; s > 0; s >>= 1) e += __shfl_xor_sync(0xFFFFFFFFu, e, s);
-  if (lane == 0) ws.scene[6] = e * (1.0f / 96.0f);
+  st.extent = e * (1.0f / 96.0f);
+  return st;
+}
+
+__device__ __forceinline__ void warp_scene(const BvhView& bvh, const WarpStack& ws) {
+  if (!bvh.has_root) return;
+  const SceneStats st = scene_stats(bvh);
+  if ((threadIdx.x & 31) == 0) {
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      ws.scene[a] = st.lo[a];
+      ws.scene[3 + a] = st.hi[a];
+    }
+    ws.scene[6] = st.extent;
+  }
   __syncwarp();
 }
 
@@ -2287,13 +2302,40 @@ struct VarShader {
 
 // Bent and sampled rays share no direction: they are traced as pairs
 // (environment lighting with 8 samples, 100k triangles, 400 x 400: 3.25 ms a ray
-// a lane, 1.70 as pairs; 2.1 at 5 blocks per SM, 2.4 at 6, which spill).
+// a lane, 1.70 as pairs; 2.1 at 5 blocks per SM, 2.4 at 6, which spill). But most
+// rays of an image miss the sphere, and pinhole rays that visit few nodes each gain
+// nothing from being paired; once the image fills the chip, a ray a lane is faster on
+// small trees. A ray a lane against pairs (ms), clouds of small triangles:
+//   reflect   500^2   1k 0.087 / 0.097   5k 0.138 / 0.148   20k 0.257 / 0.249
+//             800^2   1k 0.128 / 0.173   20k 0.447 / 0.508  60k 0.849 / 0.860  150k 1.58 / 1.40
+//             1080^2  1k 0.196 / 0.278   20k 0.728 / 0.879  60k 1.41 / 1.51    150k 2.65 / 2.46
+//   lighting  1080^2, 4 samples  1k 0.285 / 0.345  5k 0.558 / 0.604  20k 1.10 / 1.04
+//             1080^2, 8 samples  1k 0.421 / 0.431  5k 0.882 / 0.752
+// and below 131k pixels pairs always. Large triangles make long hit lists, for which
+// pairs are better again: refract at 1080^2, 1k 0.82 / 0.99, 5k 6.4 / 5.4 ms, with 0.6 and 3
+// hits expected a ray.
+constexpr int kVariantStack = 16;
+__device__ __forceinline__ bool variant_lanes(const TraceParams& p) {
+  if (!p.bvh.has_root) return false;
+  const SceneStats st = scene_stats(p.bvh);
+  const float x = st.hi[0] - st.lo[0], y = st.hi[1] - st.lo[1], z = st.hi[2] - st.lo[2];
+  const float hits = 0.75f * (float)p.bvh.P * st.extent * st.extent / (x * y + y * z + z * x);
+  return hits < 1.0f;
+}
+// Where the sizes leave the choice to the hits to expect (p.fwd_pair), both
+// kernels are launched and one returns at once.
+template <bool kLanes>
 __global__ void __launch_bounds__(kTraceThreads, 4) k_variant(const __grid_constant__ TraceParams p) {
+  if (p.fwd_pair && variant_lanes(p) != kLanes) return;
   Counters cnt;
   VarShader sh(p);
-  unsigned char* rest;
-  const Smem sm = packet_smem<kChunk>(rest);
-  drive<0>(p, sm, sh, cnt, pair_mem(rest));
+  if constexpr (kLanes) {
+    drive<kVariantStack>(p, thread_smem<kVariantStack>(), sh, cnt);
+  } else {
+    unsigned char* rest;
+    const Smem sm = packet_smem<kChunk>(rest);
+    drive<0>(p, sm, sh, cnt, pair_mem(rest));
+  }
   add_stats(p.stats, sh.n_rays, sh.n_eval, sh.n_blend, cnt);
 }
 
@@ -3842,6 +3884,12 @@ __global__ void __launch_bounds__(kTraceThreads) k_hit_stream(HitStreamParams p)
 
 }  // namespace
 
+bool variant_may_go_by_lanes(const TraceParams& p) {
+  if (p.variant == 0) return false;
+  const long long samples = p.variant == 3 ? std::max(p.samples, 1) : 1;
+  return 32ll * p.ntiles > (1 << 17) + 10ll * p.bvh.P + 300000 * (samples - 1);
+}
+
 cudaError_t launch_zero(const ZeroList& z, cudaStream_t s) {
   size_t most = 0;
   for (int i = 0; i < z.n; ++i) most = std::max(most, (size_t)z.words[i]);
@@ -3885,7 +3933,7 @@ const void* kernel_for(int which, int cfg) {
 
 int trace_blocks_per_sm(int which, int cfg) {
   int n = 0;
-  const void* fn = which == 2 ? (const void*)k_variant : (which == 3 ? collect_fn(cfg) : kernel_for(which, cfg));
+  const void* fn = which == 2 ? (const void*)k_variant<false> : (which == 3 ? collect_fn(cfg) : kernel_for(which, cfg));
   const size_t smem = which == 2 ? pair_smem<kChunk>() : trace_smem_bytes(cfg);
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, kTraceThreads, smem) != cudaSuccess) n = 1;
   return n > 0 ? n : 1;
@@ -4001,7 +4049,8 @@ cudaError_t launch_collect(const TraceParams& in, int grid, cudaStream_t s) {
 
 cudaError_t launch_forward(const TraceParams& p, int grid, cudaStream_t s) {
   if (p.variant != 0) {
-    k_variant<<<grid, kTraceThreads, pair_smem<kChunk>(), s>>>(p);
+    if (p.fwd_pair) k_variant<true><<<grid, kTraceThreads, (size_t)kTraceThreads * (kVariantStack + kChunk) * 8, s>>>(p);
+    k_variant<false><<<grid, kTraceThreads, pair_smem<kChunk>(), s>>>(p);
     return cudaGetLastError();
   }
   switch (p.mode) {

@@ -159,7 +159,7 @@ struct TraceParams {
   int collect_queries;  // collecting pass: queries stored per ray at most (0 = all the march makes)
   int count_work;       // count node visits and triangle tests (tt_stats), off by default
   int bwd_pair;         // adjoint launched as a replay-only / traversing pair: one of the two works
-  int fwd_pair;         // shading pass of the split forward launched as such a pair
+  int fwd_pair;         // shading pass of the split forward, or a sphere program, launched as such a pair
   int parts_log;  // log2 of the parts a tile is taken in (packet drivers)
   int* work;    // tile counter, zero at launch
   int* status;  // kStatus* bits
@@ -226,6 +226,9 @@ cudaError_t trace_init(int cfg, int mode);
 // Traversal-only pass that fills the hit cache with every query of the march.
 cudaError_t launch_collect(const TraceParams& p, int grid, cudaStream_t s);
 cudaError_t launch_forward(const TraceParams& p, int grid, cudaStream_t s);
+// A sphere program on an image so large, over so small a tree, that a ray a lane
+// may beat pairs of nodes and rays (p.fwd_pair: launch_forward enqueues both kernels).
+bool variant_may_go_by_lanes(const TraceParams& p);
 cudaError_t launch_backward(const TraceParams& p, int grid, cudaStream_t s);
 cudaError_t launch_hit_stream(const HitStreamParams& p, cudaStream_t s);
 // Secondary-ray passes (views[0] only): trace level p.sec.level, resolve it,
