@@ -598,7 +598,7 @@ def secondary_leg(dev, steps=3, seed=0, default_only=False):
     if not default_only:  # the schedule's two parts, each switched off once
         tr.set_sort_secondary(False)
         ms_unsorted, _ = timed()
-        tr.set_sort_secondary(True)
+        tr.set_sort_secondary(None)
         tr.set_split_forward(False)
         ms_fused, _ = timed()
         tr.set_split_forward(True)

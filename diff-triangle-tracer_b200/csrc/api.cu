@@ -235,7 +235,7 @@ int tt_set_option(tt_tracer* h, int option, int value) {
   if (!h) return TT_ERR_INVALID;
   switch (option) {
     case TT_OPT_SPLIT_FORWARD: h->split_forward = value != 0; return TT_OK;
-    case TT_OPT_SORT_SECONDARY: h->sort_secondary = value != 0 ? 1 : 0; return TT_OK;
+    case TT_OPT_SORT_SECONDARY: h->sort_secondary = value == -1 ? -1 : (value != 0 ? 1 : 0); return TT_OK;
     case TT_OPT_WORK_COUNTERS: h->count_work = value != 0; return TT_OK;
     case TT_OPT_COLLECT_QUERIES:
       TT_REQUIRE(h, value >= 0, "collect_queries must be >= 0");
@@ -903,13 +903,16 @@ int tt_forward_secondary(tt_tracer* h, const tt_fwd_args* a, const tt_secondary*
   ++h->trace_launches;
   uint32_t *keys = nullptr, *vals = nullptr, *keys2 = nullptr, *vals2 = nullptr, *hist = nullptr;
   // Pairs of (node, ray) leave a warp little to gain from neighbouring rays; what
-  // the sort still saves is L2 misses, and it costs four passes a level. A step,
-  // sorted against in spawn order (ms): 20k triangles, 203 x 151 pixels 0.45 /
-  // 0.34, 1024 x 1024 1.13 / 0.93; 500k, 256 x 256 4.3 / 3.2, 800 x 800 10.3 / 9.6,
-  // 1.28M pixels 17.9 / 17.6, 2.56M 33.6 / 33.8; 2M, 256 x 256 55.8 / 36.4, 1.28M
-  // 249 / 254, 2.56M 465 / 514.
-  constexpr long long kSortPixels = 1 << 20;
-  const bool sorts = h->sort_secondary < 0 ? R > kSortPixels : h->sort_secondary != 0;
+  // the sort still saves is L2 misses, of many rays in a large tree, and it costs four
+  // passes a level. A step, sorted against in spawn order (ms):
+  //   20k triangles    1.05M pixels 1.48 / 1.04, 2.56M 2.74 / 2.05
+  //   200k             1.31M 5.57 / 5.11, 2.56M 11.3 / 10.6
+  //   500k             1.05M 14.5 / 14.4, 1.28M 14.3 / 14.1, 2.07M 16.6 / 16.5, 2.56M 30.8 / 31.5
+  //   1M               0.64M 49.6 / 52.0, 1.05M 72.0 / 79.6, 2.07M 38.8 / 39.5, 2.56M 149 / 178
+  //   2M               0.26M 79.3 / 70.4, 0.64M 140 / 145, 1.28M 186 / 202, 2.56M 419 / 493
+  //   3M               0.26M 123 / 105
+  constexpr double kSortWork = 549755813888.0;  // 2^39 triangles x pixels
+  const bool sorts = h->sort_secondary < 0 ? (double)R * (double)a->P > kSortWork : h->sort_secondary != 0;
   if (sorts && sec->max_depth > 0) {
     const long long cap = R << sec->max_depth;  // the deepest level's capacity
     const size_t hw = tt::sort_pairs_hist_words((int)cap);

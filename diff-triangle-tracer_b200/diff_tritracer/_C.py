@@ -416,11 +416,12 @@ class OptixTracer:
         the counts cost the packet traversal ~4 % of its time)."""
         check(self._h, lib.tt_set_option(self._h, _lib.TT_OPT_WORK_COUNTERS, 1 if on else 0))
 
-    def set_sort_secondary(self, on: bool = True):
+    def set_sort_secondary(self, on: bool | None = True):
         """Trace each level of spawned secondary rays sorted by direction
-        (octahedral bins) and origin, or in spawn order (False). Until this is
-        called, images of more than 2^20 pixels sort. The results are the same."""
-        check(self._h, lib.tt_set_option(self._h, _lib.TT_OPT_SORT_SECONDARY, 1 if on else 0))
+        (octahedral bins) and origin (True), in spawn order (False), or as the
+        number of triangles times pixels suggests (None; until this is called).
+        The results are the same."""
+        check(self._h, lib.tt_set_option(self._h, _lib.TT_OPT_SORT_SECONDARY, -1 if on is None else (1 if on else 0)))
 
     def _scene_fwd_args(self, triangles_points, sigma, num_points_per_triangle, cumsum_of_points_per_triangle,
                         number_of_points, shs, sh_degree, opacities, scaling, density_factor, bg_color,

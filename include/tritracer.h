@@ -249,11 +249,11 @@ int tt_set_traversal(tt_tracer* h, int traversal, int k, int stack_depth);
  *   replays them. The first needs far fewer registers, so more warps hide
  *   the latency of the node and triangle loads. 0: one fused kernel that
  *   traverses and shades.
- * TT_OPT_SORT_SECONDARY, 1 (default above 2^20 pixels): the secondary-ray passes
- *   trace each level of spawned rays in order of direction (octahedral bins) and origin (Morton
+ * TT_OPT_SORT_SECONDARY, 1: the secondary-ray passes trace each level of
+ *   spawned rays in order of direction (octahedral bins) and origin (Morton
  *   code), after a radix sort of the level, so the rays of a warp cross
- *   nearly the same BVH nodes. 0 (default up to 2^20 pixels): in the order they were
- *   spawned.
+ *   nearly the same BVH nodes. 0: in the order they were spawned. -1 (default):
+ *   1 where triangles times pixels exceed 2^39, else 0.
  * TT_OPT_COLLECT_QUERIES, n >= 0 (default 2): the traversal-only pass of the
  *   split forward stores at most n k-closest queries per ray (0: every query
  *   of the march, also those past the point where the ray's transmittance
