@@ -1,6 +1,7 @@
 // C ABI (include/tritracer.h): the handle that replaces the reference's
 // OptixTracer class (tritracer/tracer.h:67-126, tracer.cpp, pipeline.cpp).
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -140,8 +141,11 @@ long long cache_pool_cap_colors(int k, long long rays, size_t bytes) {
   return (long long)(cap < 0xFFFFFFF0ull ? cap : 0xFFFFFFF0ull);
 }
 
-// Colour rows of a plain cache with `cap` pool entries (after the pool's keys).
+// Colour rows of a plain cache with `cap` pool entries (after the pool's keys). The
+// kernels stride over three floats an entry in an int: a cache beyond that (328
+// bytes a ray and 336 a pool entry at k = 16: 230 GB) goes without.
 float* cache_colors_of(void* cache, int k, long long rays, long long cap) {
+  if (3 * std::max(rays, cap) > INT_MAX) return nullptr;
   return reinterpret_cast<float*>(static_cast<char*>(cache) + tt::hit_cache_main_bytes(k, rays) +
                                   (size_t)(k + 2) * 8 * (size_t)cap);
 }

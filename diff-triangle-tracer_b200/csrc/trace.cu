@@ -1523,8 +1523,7 @@ __device__ __forceinline__ bool cache_colors_on(const TraceParams& p) {
   return p.cache_mode != kCacheRead || (cache_header_ptr(p)->k & kCacheColorsFlag) != 0u;
 }
 // Colours of the main-part entry of ray g or of pool entry e (slot i's three
-// channels at i * stride). Three times either count fits an int: every entry
-// takes over 400 bytes of the buffer.
+// channels at i * stride). Three times either count fits an int, or there are no rows.
 template <int K>
 __device__ __forceinline__ float* cache_color_rows(const TraceParams& p, bool main_part, long long g, uint32_t e,
                                                    int& stride) {
