@@ -432,7 +432,7 @@ __device__ __forceinline__ bool test_pairs(const RayW& r, unsigned long long key
   const float far = __shfl_sync(full, tmax, ray);
   unsigned long long key = kEmptyKey;
   float t = 0.f;
-  const bool meets = have && isect_tri_p(q, PermRt(q.perm), a, b, c, t);
+  const bool meets = have && isect_tri(q, a, b, c, t);
   if (meets && t >= 0.f && t <= far) {
     key = hit_key(t, (uint32_t)__float_as_int(a.w));
     if (key < lo) key = kEmptyKey;
