@@ -213,7 +213,7 @@ int tt_set_traversal(tt_tracer* h, int traversal, int k, int stack_depth) {
   TT_REQUIRE(h, k == 0 || k == 16 || k == 32, "k must be 16 or 32");
   TT_REQUIRE(h, stack_depth == 0 || stack_depth == 24 || stack_depth == 32, "stack_depth must be 24 or 32");
   // sphere variants bend rays incoherently: their queries take (node,
-  // ray) pairs, whatever the stack depth
+  // ray) pairs or a stack a lane of their own, whatever the stack depth
   const bool lanes = traversal == TT_TRAVERSAL_LANES || h->cfg.variant != TT_VARIANT_PLAIN;
   TT_REQUIRE(h, !(lanes && k == 32), "k = 32 needs packet traversal");
   TT_REQUIRE(h, lanes || stack_depth == 0 || stack_depth == 32, "stack_depth applies to lane traversal");

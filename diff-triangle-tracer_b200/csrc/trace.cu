@@ -275,9 +275,11 @@ __device__ __forceinline__ void query(const BvhView& bvh, const RayW& r, unsigne
 // frustum alone (104k -> 41k instructions a tile), 5.3 with the hits deferred
 // and the pairs compacted (26k), 3.9 with the seven loads of a node wave in
 // flight at once (the test's short cuts had serialised them), 3.3 with 20
-// instead of 16 warps per SM (ray data shuffled instead of in shared memory).
-// What bounds it: latency (issue slots ~50 % busy at 20 warps), the node and
-// triangle loads' from L2 first.
+// instead of 16 warps per SM (ray data shuffled instead of in shared memory); 3.4
+// with a stack that holds every scene's nodes and a count of what the frustum
+// holds (below).
+// What bounds it: issue (62 % of cycles at 20 warps) and the latencies between,
+// fixed ones and the node and triangle loads' from L2.
 //
 // The frustum lives in the axes of the rays' dominant direction z: for z' (z
 // times the sign of the directions) in [z0, z1], every ray's u lies between
@@ -2738,10 +2740,10 @@ __global__ void __launch_bounds__(kTraceThreads, kMinBlocks) k_backward(const __
 // 0.24 / 0.18 / 0.18. (Scans over the whole warp instead of a ray's lanes: 3.2 and
 // 22.1.) These are with one sum over all channels; the channels' own sums made a step
 // of the 1M triangles 9.49 instead of 9.20 ms, of the exact 200k 0.59 instead of 0.57.
-// It issues on under half of the cycles, with L2 35 and DRAM 15 % busy: bound by
+// It issues on 48 % of the cycles, with L2 38 and DRAM 15 % busy: bound by
 // instructions and their latency at 16 warps per SM. Its loop is as long as the
-// instruction cache: waits for instructions doubled (0.7 to 1.6 of ~9 cycles an
-// instruction) with the sums' chain unrolled and the SH evaluation inlined, 9.76 ms a step.
+// instruction cache: waits for instructions were 1.6 instead of 1.0 of ~9 cycles an
+// instruction with the sums' chain unrolled and the SH evaluation inlined, 9.76 ms a step.
 constexpr int kVisits = 6;
 
 // Inclusive sum over the lanes of a segment (first lane `seg`) of at most 8.
@@ -3510,9 +3512,11 @@ __global__ void __launch_bounds__(kTraceThreads, kMinBlocks) k_sec_primary(const
   add_stats(p.stats, sh.n_rays, sh.n_eval, sh.n_blend, cnt);
 }
 
-// Levels >= 1: spawned rays, incoherent: one ray per lane, with a
-// kSecStack-entry stack in shared memory per lane (continued in local
-// memory) and kSecBlocks blocks per SM.
+// Levels >= 1: spawned rays, shaded one a lane. Their queries come from the
+// traversal pass before (pairs, k_sec_collect); a query it did not store, and every
+// one with TT_OPT_SPLIT_FORWARD off, is traversed here with a kSecStack-entry
+// stack in shared memory per lane (continued in local memory), kSecBlocks blocks
+// per SM.
 #ifndef TT_SEC_STACK
 #define TT_SEC_STACK 32
 #endif
@@ -3574,10 +3578,11 @@ __global__ void __launch_bounds__(kTraceThreads, kSecCollectBlocks) k_sec_collec
 // Sort keys of the spawned rays of level p.sec.level: the direction in 16 x
 // 16 octahedral bins (8 bits) over the Morton code of the origin, 7 bits an
 // axis, within the root box of the BVH (21 bits); slots past the level's
-// count get 0xFFFFFFFF and sort after every ray. On C3 this order traces the
-// spawned levels in 29.9 ms a step against 30.7 with the direction octant
-// over a 27-bit Morton code and 32.5 with the origin first; finer direction
-// bins (1024, 4096) or coarser origins were slower.
+// count get 0xFFFFFFFF and sort after every ray. The order was chosen when these
+// rays were traversed one a lane (500k triangles, 2 views of 800^2, two bounces, a
+// step): 29.9 ms, against 30.7 with the direction octant over a 27-bit Morton code and
+// 32.5 with the origin first; finer direction bins (1024, 4096) or coarser origins
+// were slower. Pairs depend on it less (TT_OPT_SORT_SECONDARY).
 __device__ __forceinline__ uint32_t spread3(uint32_t v) {  // 9 bits -> every third of 27
   v &= 0x1FFu;
   v = (v | (v << 16)) & 0x030000FFu;

@@ -339,9 +339,11 @@ int tt_device_status(tt_tracer* h, void* stream);
 /* Counters of the handle's forward kernels since the last tt_reset_stats (no
  * reference counterpart; the reference reports only gpu_time). Evaluated hits
  * are hits at or beyond the near plane whose window function was computed;
- * blended hits are those composited; node visits (per ray), triangle tests and
- * queries (k-closest traversals) describe the traversal work (node visits and
- * triangle tests only with TT_OPT_WORK_COUNTERS on). kernel_launches counts
+ * blended hits are those composited; node visits, triangle tests and queries
+ * (k-closest traversals) describe the traversal work (node visits and
+ * triangle tests only with TT_OPT_WORK_COUNTERS on). A node that a warp packet
+ * opens counts for every ray of the packet, entered by that ray or not; a lane's
+ * or a pair's counts once. kernel_launches counts
  * every kernel this handle enqueued (BVH steps included). */
 typedef struct tt_stats {
   unsigned long long rays;
